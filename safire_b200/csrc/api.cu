@@ -93,6 +93,7 @@ struct afqmc_ham_s {
   bool coulomb_fp64 = false;  // mixed precision: EJ's Coulomb vector from a complex128 GEMM
   int mixed_ops = AFQMC_MIXED_ALL;  // which operations a mixed-precision call runs on TF32
   double* Likn = nullptr;               // [nspin_H2][M][M][Nc]
+  bool likn_sym[2] = {false, false};    // L[i][k][n] == L[k][i][n] bit for bit, per spin block
   c128* Lnak[2] = {nullptr, nullptr};   // [Nc][nel_s][M]
   double* Lnak_r[2] = {nullptr, nullptr};
   c128* haj = nullptr;                  // [nel_tot][M]
@@ -419,6 +420,19 @@ __global__ void lnak_reorder_kernel(const c128* __restrict__ in, c128* __restric
   if (out_r) out_r[o] = v.x;
 }
 
+// *differ is set when some L[i][k][n] and L[k][i][n] differ in a bit; one CTA per pair (i, k)
+__global__ void __launch_bounds__(128) asymmetry_kernel(const double* __restrict__ L, int M, int Nc,
+                                                        int* differ) {
+  const int i = blockIdx.y, k = blockIdx.x;
+  if (i >= k) return;
+  const double* a = L + (long(i) * M + k) * Nc;
+  const double* b = L + (long(k) * M + i) * Nc;
+  bool d = false;
+  for (int n = threadIdx.x; n < Nc; n += blockDim.x)
+    d = d || __double_as_longlong(a[n]) != __double_as_longlong(b[n]);
+  if (d) *differ = 1;
+}
+
 }  // namespace api_kernels
 
 namespace {
@@ -455,7 +469,10 @@ int ham_vhs(afqmc_ham_s* h, cudaStream_t s, const c128* X, c128* V, int W, doubl
     p.B = h->Likn + size_t(is % h->nspin_H2) * MM * h->Nc; p.ldb = h->Nc; p.strideB = 0;
     p.C = V + size_t(is) * W * MM; p.ldc = MM; p.strideC = 0;
     p.alpha = cmk(std::sqrt(dt), 0); p.beta = cmk(0, 0);
-    AFQMC_TRY(zgemm(s, 1, GN, false, GT, true, p));
+    if (h->likn_sym[is % h->nspin_H2])
+      AFQMC_TRY(zgemm_sym_pairs(s, h->M, p));
+    else
+      AFQMC_TRY(zgemm(s, 1, GN, false, GT, true, p));
   }
   return AFQMC_OK;
 }
@@ -640,23 +657,35 @@ extern "C" int afqmc_ham_create(int walker_type, int M, int nup, int ndn, int Nc
   }
   // v0[i][l] = -1/2 sum_{j,n} L[i][j][n] L[l][j][n]  (host copy, as the reference keeps it)
   {
-    c128* v0 = nullptr;
-    AFQMC_TRY(dalloc(&v0, size_t(nspin_H2) * MM));
+    c128* v0 = nullptr;  // and, behind it, the asymmetry flags of the spin blocks
+    AFQMC_TRY(dalloc(&v0, size_t(nspin_H2) * MM + 1));
+    int* differ_d = reinterpret_cast<int*>(v0 + size_t(nspin_H2) * MM);
+    cudaMemsetAsync(differ_d, 0, 2 * sizeof(int), s);
+    for (int isp = 0; isp < nspin_H2 && M <= 65535; ++isp)
+      api_kernels::asymmetry_kernel<<<dim3(M, M), 128, 0, s>>>(h->Likn + size_t(isp) * MM * Nc, M,
+                                                              Nc, differ_d + isp);
+    int st = launch_status("asymmetry_kernel");
     h->vexx_h.assign(size_t(nspin_H2) * MM, 0.0);
-    std::vector<c128> tmp(static_cast<size_t>(MM));
-    for (int isp = 0; isp < nspin_H2; ++isp) {
+    for (int isp = 0; isp < nspin_H2 && !st; ++isp) {
       GemmParams p{};
       p.m = M; p.n = M; p.k = int(long(M) * Nc);
       p.A = h->Likn + size_t(isp) * MM * Nc; p.lda = long(M) * Nc;
       p.B = h->Likn + size_t(isp) * MM * Nc; p.ldb = long(M) * Nc;
       p.C = v0 + size_t(isp) * MM; p.ldc = M;
       p.alpha = cmk(-0.5, 0); p.beta = cmk(0, 0);
-      int st = zgemm(s, 1, GN, true, GT, true, p);
-      if (st) { dfree(v0); return st; }
-      cudaMemcpy(tmp.data(), v0 + size_t(isp) * MM, sizeof(c128) * MM, cudaMemcpyDeviceToHost);
-      for (long e = 0; e < MM; ++e) h->vexx_h[size_t(isp) * MM + e] = tmp[e].x;
+      st = zgemm(s, 1, GN, true, GT, true, p);
     }
+    std::vector<c128> tmp(size_t(nspin_H2) * MM + 1);
+    cudaError_t e = cudaMemcpy(tmp.data(), v0, sizeof(c128) * tmp.size(), cudaMemcpyDeviceToHost);
     dfree(v0);
+    if (st) return st;
+    AFQMC_CUDA_TRY(e);
+    int differ[2];
+    std::memcpy(differ, &tmp.back(), sizeof(differ));
+    for (int isp = 0; isp < nspin_H2; ++isp) {
+      for (long i = 0; i < MM; ++i) h->vexx_h[isp * MM + i] = tmp[isp * MM + i].x;
+      h->likn_sym[isp] = M <= 65535 && differ[isp] == 0;
+    }
   }
   AFQMC_CUDA_TRY(cudaDeviceSynchronize());
   *out = h.release();

@@ -291,7 +291,7 @@ int thc_vhs(cudaStream_t s, ThcData* t, const c128* X, c128* V, int W, double dt
   q.B = t->XX; q.ldb = t->nu; q.strideB = 0;
   q.C = V; q.ldc = MM; q.strideC = 0;
   q.alpha = cmk(std::sqrt(dt), 0); q.beta = cmk(0, 0);
-  return zgemm(s, 1, GN, false, GT, true, q);
+  return zgemm_sym_pairs(s, t->M, q);  // X[i][u] X[k][u] is the same product either way
 }
 
 int thc_energy(cudaStream_t s, ThcData* t, const c128* G, long ldG, const c128* haj, double E0,

@@ -1,248 +1,85 @@
-// Batched complex128 GEMM on the FP64 DMMA path (mma.sync.m8n8k4.f64), see zgemm.cuh.
-//
-// Tile: BM x BN complex outputs per CTA, BK-deep k tiles staged through shared memory with a
-// register prefetch of the next tile (double-buffered shared memory, one barrier per k tile).
-// Shared-memory row pitches are padded so that the 8x4 / 4x8 DMMA fragment loads are free of
-// bank conflicts for both 16-byte (complex) and 8-byte (real) elements.
+// Shapes and dispatch of the batched complex128 GEMM (zgemm.cuh; the kernel is in
+// zgemm_kernel.cuh, its instantiations in zgemm_*.cu).
 #include "zgemm.cuh"
 
 namespace afqmc {
+namespace zg {
+
+using Launch = int (*)(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_nn(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_rn(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_nr(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_nt(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_nrt(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_tt(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_tn(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_hn(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_rrt(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_nc(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_nh(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_nrt_sym(cudaStream_t, const GemmParams&, const Shape&);
+
 namespace {
 
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
+constexpr int SMS = 148;
 
-template <bool REAL>
-struct Elem;
-template <>
-struct Elem<true> {
-  using T = double;
-};
-template <>
-struct Elem<false> {
-  using T = c128;
-};
-
-// pad (in elements) of the contiguous dimension of a shared tile
-template <bool TRANSPOSED_STORAGE, bool REAL>
-struct Pad {
-  static constexpr int value = (TRANSPOSED_STORAGE && !REAL) ? 2 : 4;
-};
-
-template <int BM, int BN, int BK, int WM_WARPS, int WN_WARPS, bool AT, bool AC, bool AR, bool BT,
-          bool BC, bool BR>
-struct Cfg {
-  static constexpr int NT = WM_WARPS * WN_WARPS * 32;
-  static constexpr int WM = BM / WM_WARPS;  // warp tile rows
-  static constexpr int WN = BN / WN_WARPS;  // warp tile cols
-  static constexpr int TM = WM / 8;
-  static constexpr int TN = WN / 8;
-  using TA = typename Elem<AR>::T;
-  using TB = typename Elem<BR>::T;
-  // A tile: AT ? [BK][BM+pa] : [BM][BK+pa]
-  static constexpr int PA = Pad<AT, AR>::value;
-  static constexpr int A_ROWS = AT ? BK : BM;
-  static constexpr int A_PITCH = (AT ? BM : BK) + PA;
-  static constexpr int A_ELEMS = A_ROWS * A_PITCH;
-  // B tile: BT ? [BN][BK+pb] : [BK][BN+pb]
-  static constexpr int PB = Pad<!BT, BR>::value;
-  static constexpr int B_ROWS = BT ? BN : BK;
-  static constexpr int B_PITCH = (BT ? BK : BN) + PB;
-  static constexpr int B_ELEMS = B_ROWS * B_PITCH;
-  static constexpr int A_PER_T = BM * BK / NT;
-  static constexpr int B_PER_T = BN * BK / NT;
-  static constexpr size_t SMEM =
-      2 * (size_t(A_ELEMS) * sizeof(TA) + size_t(B_ELEMS) * sizeof(TB));
-  static_assert(BM * BK % NT == 0 && BN * BK % NT == 0, "tile/threads mismatch");
-  static_assert(WM % 8 == 0 && WN % 8 == 0 && BK % 4 == 0, "tile granularity");
-};
-
-template <bool CONJ>
-__device__ __forceinline__ c128 ld_c(const c128* p) {
-  c128 v = __ldg(p);
-  if (CONJ) v.y = -v.y;
-  return v;
-}
-
-template <int BM, int BN, int BK, int WM_WARPS, int WN_WARPS, bool AT, bool AC, bool AR, bool BT,
-          bool BC, bool BR>
-__global__ void __launch_bounds__(WM_WARPS* WN_WARPS * 32)
-    zgemm_kernel(GemmParams p) {
-  using K = Cfg<BM, BN, BK, WM_WARPS, WN_WARPS, AT, AC, AR, BT, BC, BR>;
-  using TA = typename K::TA;
-  using TB = typename K::TB;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  TA* As = reinterpret_cast<TA*>(smem_raw);
-  TB* Bs = reinterpret_cast<TB*>(smem_raw + 2 * size_t(K::A_ELEMS) * sizeof(TA));
-
-  const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int wm0 = (warp / WN_WARPS) * K::WM;
-  const int wn0 = (warp % WN_WARPS) * K::WN;
-  const long b = blockIdx.z;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-
-  const TA* Ag = reinterpret_cast<const TA*>(p.A) + b * p.strideA;
-  const TB* Bg = reinterpret_cast<const TB*>(p.B) + b * p.strideB;
-
-  TA ra[K::A_PER_T];
-  TB rb[K::B_PER_T];
-
-  auto load_regs = [&](int k0) {
-#pragma unroll
-    for (int i = 0; i < K::A_PER_T; ++i) {
-      int e = tid + i * K::NT;
-      int row = AT ? e / BM : e / BK;
-      int col = AT ? e % BM : e % BK;
-      int mm = AT ? col : row, kk = AT ? row : col;
-      bool in = (m0 + mm < p.m) && (k0 + kk < p.k);
-      long off = AT ? long(k0 + kk) * p.lda + (m0 + mm) : long(m0 + mm) * p.lda + (k0 + kk);
-      if constexpr (AR) {
-        ra[i] = in ? __ldg(Ag + off) : 0.0;
-      } else {
-        ra[i] = in ? ld_c<AC>(Ag + off) : cmk(0.0, 0.0);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < K::B_PER_T; ++i) {
-      int e = tid + i * K::NT;
-      int row = BT ? e / BK : e / BN;
-      int col = BT ? e % BK : e % BN;
-      int nn = BT ? row : col, kk = BT ? col : row;
-      bool in = (n0 + nn < p.n) && (k0 + kk < p.k);
-      long off = BT ? long(n0 + nn) * p.ldb + (k0 + kk) : long(k0 + kk) * p.ldb + (n0 + nn);
-      if constexpr (BR) {
-        rb[i] = in ? __ldg(Bg + off) : 0.0;
-      } else {
-        rb[i] = in ? ld_c<BC>(Bg + off) : cmk(0.0, 0.0);
-      }
-    }
-  };
-  auto store_regs = [&](int buf) {
-    TA* as = As + buf * K::A_ELEMS;
-    TB* bs = Bs + buf * K::B_ELEMS;
-#pragma unroll
-    for (int i = 0; i < K::A_PER_T; ++i) {
-      int e = tid + i * K::NT;
-      int row = AT ? e / BM : e / BK;
-      int col = AT ? e % BM : e % BK;
-      as[row * K::A_PITCH + col] = ra[i];
-    }
-#pragma unroll
-    for (int i = 0; i < K::B_PER_T; ++i) {
-      int e = tid + i * K::NT;
-      int row = BT ? e / BK : e / BN;
-      int col = BT ? e % BK : e % BN;
-      bs[row * K::B_PITCH + col] = rb[i];
-    }
-  };
-
-  double accr[K::TM][K::TN][2], acci[K::TM][K::TN][2];
-#pragma unroll
-  for (int i = 0; i < K::TM; ++i)
-#pragma unroll
-    for (int j = 0; j < K::TN; ++j) accr[i][j][0] = accr[i][j][1] = acci[i][j][0] = acci[i][j][1] = 0.0;
-
-  const int ktiles = (p.k + BK - 1) / BK;
-  load_regs(0);
-  store_regs(0);
-  __syncthreads();
-
-  for (int kt = 0; kt < ktiles; ++kt) {
-    const int buf = kt & 1;
-    if (kt + 1 < ktiles) load_regs((kt + 1) * BK);
-    const TA* as = As + buf * K::A_ELEMS;
-    const TB* bs = Bs + buf * K::B_ELEMS;
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      TA fa[K::TM];
-      TB fb[K::TN];
-#pragma unroll
-      for (int i = 0; i < K::TM; ++i) {
-        int r = wm0 + i * 8 + g, c = kk + t;
-        fa[i] = AT ? as[c * K::A_PITCH + r] : as[r * K::A_PITCH + c];
-      }
-#pragma unroll
-      for (int j = 0; j < K::TN; ++j) {
-        int cn = wn0 + j * 8 + g, r = kk + t;
-        fb[j] = BT ? bs[cn * K::B_PITCH + r] : bs[r * K::B_PITCH + cn];
-      }
-#pragma unroll
-      for (int i = 0; i < K::TM; ++i) {
-#pragma unroll
-        for (int j = 0; j < K::TN; ++j) {
-          if constexpr (AR && BR) {
-            dmma(accr[i][j][0], accr[i][j][1], fa[i], fb[j]);
-          } else if constexpr (AR) {
-            dmma(accr[i][j][0], accr[i][j][1], fa[i], fb[j].x);
-            dmma(acci[i][j][0], acci[i][j][1], fa[i], fb[j].y);
-          } else if constexpr (BR) {
-            dmma(accr[i][j][0], accr[i][j][1], fa[i].x, fb[j]);
-            dmma(acci[i][j][0], acci[i][j][1], fa[i].y, fb[j]);
-          } else {
-            dmma(accr[i][j][0], accr[i][j][1], fa[i].x, fb[j].x);
-            dmma(accr[i][j][0], accr[i][j][1], -fa[i].y, fb[j].y);
-            dmma(acci[i][j][0], acci[i][j][1], fa[i].x, fb[j].y);
-            dmma(acci[i][j][0], acci[i][j][1], fa[i].y, fb[j].x);
-          }
-        }
-      }
-    }
-    if (kt + 1 < ktiles) store_regs(buf ^ 1);
-    __syncthreads();
-  }
-
-  // epilogue
-  c128* Cg = p.C + b * p.strideC;
-  c128* Dg = p.D ? p.D + b * p.strideD : nullptr;
-  const bool use_beta = (p.beta.x != 0.0 || p.beta.y != 0.0);
-#pragma unroll
-  for (int i = 0; i < K::TM; ++i) {
-    int row = m0 + wm0 + i * 8 + g;
-    if (row >= p.m) continue;
-#pragma unroll
-    for (int j = 0; j < K::TN; ++j) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        int col = n0 + wn0 + j * 8 + 2 * t + h;
-        if (col >= p.n) continue;
-        c128 v = cmul(p.alpha, cmk(accr[i][j][h], acci[i][j][h]));
-        long oc = long(row) * p.ldc + col;
-        if (use_beta) v = cadd(v, cmul(p.beta, Cg[oc]));
-        Cg[oc] = v;
-        if (Dg) {
-          long od = long(row) * p.ldd + col;
-          Dg[od] = p.d_store ? v : cadd(Dg[od], v);
-        }
-      }
+// Columns of a tile in units of 8, at most 8 of them: the number that pads n least, where a
+// narrower tile has to save 1/32 of the work per unit given up (it reads A that much more often).
+int fit_cols(int n) {
+  const int need = ceil_div(n, 8);
+  if (need <= 8) return need;
+  int best = 8;
+  long cost = long(ceil_div(need, 8)) * 8 * 32;
+  for (int c = 7; c >= 4; --c) {
+    const long q = long(ceil_div(need, c)) * c * (32 + 8 - c);
+    if (q < cost) {
+      cost = q;
+      best = c;
     }
   }
+  return best;
 }
 
-template <int BM, int BN, int BK, int WMW, int WNW, bool AT, bool AC, bool AR, bool BT, bool BC,
-          bool BR>
-int launch(cudaStream_t s, int batch, const GemmParams& p) {
-  using K = Cfg<BM, BN, BK, WMW, WNW, AT, AC, AR, BT, BC, BR>;
-  auto kern = zgemm_kernel<BM, BN, BK, WMW, WNW, AT, AC, AR, BT, BC, BR>;
-  AFQMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(K::SMEM)));
-  dim3 grid(ceil_div(p.n, BN), ceil_div(p.m, BM), batch);
-  kern<<<grid, K::NT, K::SMEM, s>>>(p);
-  return launch_status("zgemm_kernel");
-}
-
-template <bool AT, bool AC, bool AR, bool BT, bool BC, bool BR>
-int launch_cfg(cudaStream_t s, int batch, const GemmParams& p) {
-  // small problems (per-walker products with N ~ 50) use a 32-row tile to cut padding waste
-  if (p.m <= 32) return launch<32, 64, 16, 1, 4, AT, AC, AR, BT, BC, BR>(s, batch, p);
-  return launch<64, 64, 16, 2, 4, AT, AC, AR, BT, BC, BR>(s, batch, p);
+// Warps (8-row strips) of a tile.  The FP64 tensor path belongs to the SM's four schedulers, and a
+// CTA's warp i runs on scheduler i mod 4 whatever else is resident: 5 strips take the time of 8
+// (m=200, n=50, k=200, 1024 problems: 813 us with 5 warps, which divide 200, 678 us with 4,
+// 749 us with 8).  So strips count in groups of four; four warps read B twice as often as eight,
+// which costs them about 1/16.
+int fit_rows(int m) {
+  const int need = ceil_div(m, 8);
+  if (need <= 8) return need;
+  const long four = long(ceil_div(need, 4)) * 4 * 17, eight = long(ceil_div(need, 8)) * 8 * 16;
+  if (four < eight) return 4;
+  for (int w = 5; w < 8; ++w)  // the same number of tiles with less padding to load
+    if (ceil_div(need, w) == ceil_div(need, 8)) return w;
+  return 8;
 }
 
 }  // namespace
+
+// The CTA shape: tiles fitted to m and n; then, where those are too few to give every SM one, the
+// K range of a single problem split over a cluster of up to 8 CTAs (each keeping at least 8 K
+// tiles, so that the reduction stays small against the product), and the tiles halved down to 8
+// strips in all (below that the operand loads bound a tile).
+Shape shape(int batch, int m, int n, int k) {
+  Shape sh{fit_rows(m), fit_cols(n), 1};
+  auto ctas = [&] { return long(ceil_div(m, 8 * sh.warps)) * ceil_div(n, 8 * sh.tn) * batch; };
+  if (batch == 1 && ctas() < SMS) {
+    const long s = SMS / ctas(), ks = ceil_div(k, 16) / 8;
+    const long c = s < ks ? s : ks;
+    sh.split = int(c < 1 ? 1 : (c > 8 ? 8 : c));
+  }
+  while (ctas() * sh.split < SMS && sh.warps * sh.tn > 8) {
+    if (sh.tn >= sh.warps)
+      sh.tn = (sh.tn + 1) / 2;
+    else
+      sh.warps = (sh.warps + 1) / 2;
+  }
+  if (m > 65535l * 8 * sh.warps) sh.warps = 8;  // grid.y limit
+  return sh;
+}
+
+}  // namespace zg
 
 int zgemm(cudaStream_t s, int batch, GemmTrans ta, bool a_real, GemmTrans tb, bool b_real,
           const GemmParams& p) {
@@ -262,24 +99,43 @@ int zgemm(cudaStream_t s, int batch, GemmTrans ta, bool a_real, GemmTrans tb, bo
     return zgemm(s, batch, AT ? GT : GN, a_real, BT ? GT : GN, b_real, p);
   }
   // Instantiated combinations (the products the walker step and its setup use).
-#define AFQMC_GEMM_CASE(at, ac, ar, bt, bc, br)                                    \
-  if (AT == at && AC == ac && a_real == ar && BT == bt && BC == bc && b_real == br) \
-    return launch_cfg<at, ac, ar, bt, bc, br>(s, batch, p);
-  AFQMC_GEMM_CASE(false, false, false, false, false, false)  // A*B
-  AFQMC_GEMM_CASE(false, false, true, false, false, false)   // real A * B
-  AFQMC_GEMM_CASE(false, false, false, false, false, true)   // A * real B
-  AFQMC_GEMM_CASE(false, false, false, true, false, false)   // A * B^T
-  AFQMC_GEMM_CASE(false, false, false, true, false, true)    // A * real B^T
-  AFQMC_GEMM_CASE(true, false, false, true, false, false)    // A^T * B^T
-  AFQMC_GEMM_CASE(true, false, false, false, false, false)   // A^T * B
-  AFQMC_GEMM_CASE(true, true, false, false, false, false)    // A^H * B
-  AFQMC_GEMM_CASE(false, false, true, true, false, true)     // real A * real B^T
-  AFQMC_GEMM_CASE(false, false, false, false, true, false)   // A * conj(B)
-  AFQMC_GEMM_CASE(false, false, false, true, true, false)    // A * B^H
+  zg::Launch fn = nullptr;
+#define AFQMC_GEMM_CASE(at, ac, ar, bt, bc, br, name) \
+  if (AT == at && AC == ac && a_real == ar && BT == bt && BC == bc && b_real == br) fn = zg::name;
+  AFQMC_GEMM_CASE(false, false, false, false, false, false, launch_nn)  // A*B
+  AFQMC_GEMM_CASE(false, false, true, false, false, false, launch_rn)   // real A * B
+  AFQMC_GEMM_CASE(false, false, false, false, false, true, launch_nr)   // A * real B
+  AFQMC_GEMM_CASE(false, false, false, true, false, false, launch_nt)   // A * B^T
+  AFQMC_GEMM_CASE(false, false, false, true, false, true, launch_nrt)   // A * real B^T
+  AFQMC_GEMM_CASE(true, false, false, true, false, false, launch_tt)    // A^T * B^T
+  AFQMC_GEMM_CASE(true, false, false, false, false, false, launch_tn)   // A^T * B
+  AFQMC_GEMM_CASE(true, true, false, false, false, false, launch_hn)    // A^H * B
+  AFQMC_GEMM_CASE(false, false, true, true, false, true, launch_rrt)    // real A * real B^T
+  AFQMC_GEMM_CASE(false, false, false, false, true, false, launch_nc)   // A * conj(B)
+  AFQMC_GEMM_CASE(false, false, false, true, true, false, launch_nh)    // A * B^H
 #undef AFQMC_GEMM_CASE
-  set_error_detail("zgemm: operand combination (ta=%d a_real=%d tb=%d b_real=%d) not instantiated",
-                   int(ta), int(a_real), int(tb), int(b_real));
-  return AFQMC_ERR_UNSUPPORTED;
+  if (!fn) {
+    set_error_detail(
+        "zgemm: operand combination (ta=%d a_real=%d tb=%d b_real=%d) not instantiated", int(ta),
+        int(a_real), int(tb), int(b_real));
+    return AFQMC_ERR_UNSUPPORTED;
+  }
+  return fn(s, batch, p, zg::shape(batch, p.m, p.n, p.k));
+}
+
+int zgemm_sym_pairs(cudaStream_t s, int M, const GemmParams& p) {
+  if (p.m <= 0 || M <= 0) return AFQMC_OK;
+  GemmParams q = p;
+  q.sym_m = M;
+  q.n = M * M;
+  // Worth it once the blocks fill the SMs twice over: below that the time is one tile's, and the
+  // general form's tiles can be narrower than the 64 pairs of a block.  (1024 walkers, M = 200,
+  // 1600 vectors: 4.73 ms, against 8.6 ms for all pairs.)
+  const long nb = ceil_div(M, 8), blocks = nb * (nb + 1) / 2;
+  if (ceil_div(p.m, 64) * blocks < 2 * zg::SMS) return zgemm(s, 1, GN, false, GT, true, q);
+  zg::Shape sh{zg::fit_rows(p.m), 8, 1};
+  if (p.m > 65535l * 8 * sh.warps) sh.warps = 8;
+  return zg::launch_nrt_sym(s, q, sh);
 }
 
 }  // namespace afqmc

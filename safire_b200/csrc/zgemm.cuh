@@ -22,6 +22,7 @@ struct GemmParams {
   c128 alpha, beta;
   c128* D; long ldd, strideD;  // optional second output (nullptr: none)
   bool d_store;                 // D = result (true) or D += result (false)
+  int sym_m;                    // zgemm_sym_pairs only
 };
 
 // op codes for the C++ launcher
@@ -31,5 +32,18 @@ enum GemmTrans : int { GN = 0, GT = 1, GC = 2, GH = 3 };  // N, T, conj, conj-tr
 // a_real / b_real: the operand is float64 instead of complex128.
 int zgemm(cudaStream_t stream, int batch, GemmTrans ta, bool a_real, GemmTrans tb, bool b_real,
           const GemmParams& p);
+
+// C[w][(i, k)] = alpha * sum_n A[w][n] B[(i, k)][n] over all pairs of an M x M matrix (n = M*M,
+// ldc >= M*M) for a real B with B[(i, k)] == B[(k, i)] bit for bit: the pairs are computed once
+// per 8 x 8 block with block(i) <= block(k) and written to both places.  The same values as
+// zgemm(stream, 1, GN, false, GT, true, p), bit for bit.
+int zgemm_sym_pairs(cudaStream_t stream, int M, const GemmParams& p);
+
+namespace zg {
+// CTA shape of a launch: warps (8 output rows each), tn (8 output columns each), K split
+struct Shape {
+  int warps, tn, split;
+};
+}  // namespace zg
 
 }  // namespace afqmc

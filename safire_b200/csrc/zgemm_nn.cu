@@ -1,0 +1,14 @@
+// Instantiations of the DMMA GEMM kernel (one group of operand combinations per file, so that they
+// compile in parallel).
+#include "zgemm_kernel.cuh"
+
+namespace afqmc {
+namespace zg {
+
+// A*B
+int launch_nn(cudaStream_t s, int batch, const GemmParams& p, const Shape& sh) {
+  return launch_tn<Op<false, false, false, false, false, false>>(s, batch, p, sh);
+}
+
+}  // namespace zg
+}  // namespace afqmc

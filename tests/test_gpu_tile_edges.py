@@ -1,0 +1,49 @@
+"""Sizes at which the kernels change tile, register or thread layout, against numpy or complex128.
+
+The bounds are rounding bounds: eps = 2^-53 times the length of the sums and the condition or
+magnitude of the operands, with a factor of a few tens for the constant."""
+import numpy as np
+import pytest
+import torch
+
+from tests.gpu_helpers import rand_c, to_dev, to_host
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -53
+
+
+def _ham(M, N, Nc, L):
+    from safire_b200 import afqmc as A
+    _, orb = np.linalg.eigh(np.diag(np.arange(M, dtype=float)) + 0.1)
+    return A.HamiltonianOperations(A.CLOSED, M, N, N, L[None], np.eye(M)[None].astype(complex),
+                                   0.0, [orb[:, :N].T.astype(complex)])
+
+
+@pytest.mark.parametrize("W,M,Nc", [(1, 5, 3), (9, 8, 16), (33, 17, 40), (64, 32, 260), (257, 30, 37),
+                                    (256, 100, 21), (300, 41, 19)])
+def test_vhs_vbias_shapes(cuda, W, M, Nc):
+    """vbias and vHS of symmetric vectors (pairs computed once where that pays) and of vectors
+    with one bit of one element changed (every pair computed): the other elements are the same
+    bit for bit."""
+    from safire_b200 import afqmc as A
+    rs = np.random.default_rng(W)
+    N = max(1, M // 4)
+    L = rs.standard_normal((M, M, Nc))
+    L = L + L.transpose(1, 0, 2)
+    X, G = rand_c(rs, W, Nc), rand_c(rs, W, N * M)
+    ham = _ham(M, N, Nc, L)
+    V = to_host(ham.vHS(to_dev(X), 0.01))[0].reshape(W, M * M)
+    want = 0.1 * (X.real @ L.reshape(M * M, Nc).T + 1j * (X.imag @ L.reshape(M * M, Nc).T))
+    scale = 0.1 * np.max(np.abs(X)) * np.max(np.abs(L))
+    assert np.max(np.abs(V - want)) < 20 * Nc * EPS * scale
+    L2 = L.copy()
+    L2[0, 1, 0] = np.nextafter(L2[0, 1, 0], 1e9)
+    V2 = to_host(_ham(M, N, Nc, L2).vHS(to_dev(X), 0.01))[0].reshape(W, M * M)
+    keep = np.arange(M * M) != 1
+    assert np.array_equal(V[:, keep], V2[:, keep])
+    Lnak = ham.tensors().Lnak[0].real.reshape(Nc, N * M)
+    v = torch.zeros((W, Nc), dtype=torch.complex128, device=cuda)
+    ham.vbias(to_dev(G), v, 0.01)
+    want = 0.2 * (G.real @ Lnak.T + 1j * (G.imag @ Lnak.T))
+    scale = 0.2 * np.max(np.abs(G)) * np.max(np.abs(Lnak))
+    assert np.max(np.abs(to_host(v) - want)) < 20 * N * M * EPS * scale
