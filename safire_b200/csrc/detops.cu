@@ -5,6 +5,7 @@
 // MixedDensityMatrix 535-601, inverse_logdet 43-111), determinants_impl.hpp (log-det conventions),
 // propagate.hpp (apply_expM 41-70, propagate_impl 238-298), orthogonalize.hpp (131-169).
 #include "detops.cuh"
+#include "dmma.cuh"
 #include "zgemm.cuh"
 
 namespace afqmc {
@@ -167,9 +168,153 @@ __global__ void __launch_bounds__(GJ_THREADS) gj_logdet_kernel(const c128* __res
 }
 
 // ---------------------------------------------------------------------------------------------
-// Register-resident Gauss-Jordan / LU for N <= 64 (the production sizes).  One CTA of 64 C threads
-// per matrix (C = 2 column classes up to N = 32, else 4); thread t holds row
-// i = t % 64 and the columns j = h + C q of class h = t / 64 in registers (q < QMAX), so a step
+// Warp-resident Gauss-Jordan / LU for N <= 16: G lanes (the power of two >= N) hold one matrix, a
+// row per lane and its columns in registers, 32 / G matrices to a warp, no block barriers.
+// Partial pivoting as izamax; the pivots give the log determinant, the in-place Gauss-Jordan the
+// inverse.  Row interchanges move no data: each lane knows the logical index of its row.  The columns are kept rotated so that the pivot column of every step is register 0
+// (the update of column j writes register j - 1, and the finished column goes to register
+// NC - 1), so the step loop is not unrolled over k and no register index depends on N; the NC - N
+// registers past the matrix rotate along as zeros that nothing reads.  The pivot row reaches the
+// other lanes by shuffles (G <= 8) or through a shared-memory row.
+// What bounds it is the latency of the N dependent steps; small matrices are many (a trial of 34
+// determinants inverts 52224 of 3 x 3 per spin and step), so the point is matrices in flight: a
+// 128-thread CTA per matrix took 232 us for those, this form 10.4.
+// ---------------------------------------------------------------------------------------------
+constexpr int GW_WARPS = 4;
+
+template <int G, int NC, bool INVERT>
+__global__ void __launch_bounds__(32 * GW_WARPS)
+    gj_warp_kernel(const c128* __restrict__ A, long strideA, c128* Ainv, long strideInv,
+                   c128* __restrict__ ovlp, int W, int N, c128 post_scale, c128 post_add) {
+  static_assert(NC <= G, "a row per lane");
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr bool SMEM_ROW = G > 8;
+  __shared__ c128 rows[SMEM_ROW ? GW_WARPS : 1][2][SMEM_ROW ? 32 : 1];  // [warp][parity][group, column]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = lane & (G - 1), grp = lane & ~(G - 1);  // lane in the group, its first lane
+  const long w = (long(blockIdx.x) * (blockDim.x >> 5) + warp) * (32 / G) + lane / G;
+  const bool mat_ok = w < W, row_ok = mat_ok && i < N;
+  const c128* Aw = A + (mat_ok ? w : 0) * strideA + long(i) * N;
+
+  c128 a[NC];
+#pragma unroll
+  for (int j = 0; j < NC; ++j) a[j] = (row_ok && j < N) ? Aw[j] : cmk(0.0, 0.0);
+  int r = i;               // logical row
+  c128 piv_i = cmk(1, 0);  // lane k keeps pivot k and its row
+  int perm_i = i;
+  bool singular = false;
+
+  for (int k = 0; k < N; ++k) {
+    const c128 f = a[0];
+    // pivot: first max |re|+|im| over the logical rows k..N-1 (NaN counts as 0)
+    const bool cand = row_ok && r >= k;
+    const double v = cand ? cabs1(f) : 0.0;
+    unsigned long long key = (v == v) ? static_cast<unsigned long long>(__double_as_longlong(v)) : 0ull;
+    unsigned id = cand ? unsigned(r) * 32u + unsigned(lane) : 0xffffffffu;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+      const unsigned long long ok = __shfl_xor_sync(FULL, key, o);
+      const unsigned oid = __shfl_xor_sync(FULL, id, o);
+      if (ok > key || (ok == key && oid < id)) {
+        key = ok;
+        id = oid;
+      }
+    }
+    const bool zero = key == 0ull;
+    // a zero (or NaN) column: zero pivot at row k, no interchange; the candidates of a zero key
+    // tie, so the first of them is row k itself
+    const int pl = mat_ok ? int(id & 31u) : lane, p = mat_ok ? int(id >> 5) : 0;
+    const c128 piv = cmk(__shfl_sync(FULL, f.x, pl), __shfl_sync(FULL, f.y, pl));
+    const double rden = 1.0 / (piv.x * piv.x + piv.y * piv.y);
+    const c128 dinv = cmk(piv.x * rden, -piv.y * rden);
+    if (i == k) {
+      piv_i = piv;
+      perm_i = p;
+    }
+    singular = singular || zero;
+    const bool is_piv = lane == pl;
+    c128* row = nullptr;
+    if constexpr (SMEM_ROW) {
+      row = rows[warp][k & 1] + grp;
+      if (is_piv) {
+#pragma unroll
+        for (int j = 1; j < NC; ++j) row[j] = a[j];
+      }
+      __syncwarp();
+    }
+    // logical rows after the interchange
+    if (is_piv)
+      r = k;
+    else if (r == k)
+      r = p;
+    const c128 gg = cmul(f, dinv), ng = cmk(-gg.x, -gg.y);
+    const bool upd = !zero && !is_piv && (INVERT || r > k);
+    const bool scl = !zero && is_piv && INVERT;
+#pragma unroll
+    for (int j = 1; j < NC; ++j) {
+      c128 x;
+      if constexpr (SMEM_ROW)
+        x = row[j];
+      else
+        x = cmk(__shfl_sync(FULL, a[j].x, pl), __shfl_sync(FULL, a[j].y, pl));
+      c128 y = a[j];
+      if (upd) {
+        y.x = fma(ng.x, x.x, fma(gg.y, x.y, y.x));
+        y.y = fma(ng.x, x.y, fma(ng.y, x.x, y.y));
+      } else if (scl) {
+        y = cmul(x, dinv);
+      }
+      a[j - 1] = y;
+    }
+    a[NC - 1] = upd ? ng : (scl ? dinv : cmk(0.0, 0.0));
+  }
+
+  // log det: sum_k log(+-U_kk + DBL_MIN) over the group
+  c128 l = cmk(0, 0);
+  if (row_ok) l = log_pivot(piv_i, perm_i != i);
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+    l.x += __shfl_xor_sync(FULL, l.x, o);
+    l.y += __shfl_xor_sync(FULL, l.y, o);
+  }
+  if (mat_ok && i == 0) ovlp[w] = cadd(cmul(post_scale, wrap_imag(cadd(ovlp[w], l))), post_add);
+  if (INVERT) {
+    // the interchanges, undone on the columns in reverse order: pos = where column i ends
+    int pos = i;
+    for (int k = N - 1; k >= 0; --k) {
+      const int q = __shfl_sync(FULL, perm_i, grp + k);
+      if (pos == k)
+        pos = q;
+      else if (pos == q)
+        pos = k;
+    }
+    c128* Iw = Ainv + (mat_ok ? w : 0) * strideInv + long(r) * N;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {  // register j holds column j - (NC - N)
+      const int col = j - (NC - N), c = __shfl_sync(FULL, pos, grp + (col > 0 ? col : 0));
+      if (row_ok && col >= 0) Iw[c] = singular ? cmk(0.0, 0.0) : a[j];
+    }
+  }
+}
+
+template <int G, int NC>
+void launch_gj_warp(cudaStream_t s, const c128* A, long strideA, c128* Ainv, long strideInv,
+                    c128* ovlp, int W, int N, bool invert, c128 post_scale, c128 post_add) {
+  // single-warp blocks until every SM has a block's worth, so that few matrices spread out
+  const int nw = ceil_div(W, 32 / G) < 148 * GW_WARPS ? 1 : GW_WARPS;
+  const int grid = ceil_div(W, nw * (32 / G));
+  if (invert)
+    gj_warp_kernel<G, NC, true><<<grid, 32 * nw, 0, s>>>(A, strideA, Ainv, strideInv, ovlp, W,
+                                                              N, post_scale, post_add);
+  else
+    gj_warp_kernel<G, NC, false><<<grid, 32 * nw, 0, s>>>(A, strideA, nullptr, 0, ovlp, W, N,
+                                                               post_scale, post_add);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Register-resident Gauss-Jordan / LU for 16 < N <= 32 (a matrix per warp was slower there: 27 x 27
+// in a warp's registers leaves too few warps an SM).  One CTA of 64 C threads per matrix (C = 2
+// column classes); thread t holds row i = t % 64 and the columns j = h + C q of class h = t / 64 in registers (q < QMAX), so a step
 // touches shared memory only for the pivot column, the pivot row and the row that moves in the
 // interchange.
 // Step k: every warp finds the pivot p (first max |re|+|im| in column k, rows k..N-1, as izamax)
@@ -184,7 +329,7 @@ __global__ void __launch_bounds__(GJ_THREADS) gj_logdet_kernel(const c128* __res
 // order).  Two barriers a step.
 // ---------------------------------------------------------------------------------------------
 template <int QMAX, int C, bool INVERT>
-__global__ void __launch_bounds__(64 * C, C == 2 ? 3 : (QMAX <= 13 ? 2 : 1)) gj_reg_kernel(const c128* __restrict__ A,
+__global__ void __launch_bounds__(64 * C, 3) gj_reg_kernel(const c128* __restrict__ A,
                                                                long strideA,
                                                                c128* __restrict__ Ainv,
                                                                long strideInv,
@@ -383,24 +528,253 @@ void launch_gj_reg(cudaStream_t s, const c128* A, long strideA, c128* Ainv, long
                                                        post_scale, post_add);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Blocked Gauss-Jordan / LU for 32 < N <= 64: one CTA of four warps per matrix, the matrix in shared
+// memory, eight columns at a time.
+//   panel     warp 0 holds the panel's columns in registers (two rows per lane) and runs eight
+//             in-place Gauss-Jordan steps on them alone: partial pivoting (first max |re|+|im|, as
+//             izamax) over the rows not yet used, no block barrier;
+//   trailing  the steps' product is the identity with the pivot rows' columns replaced by the
+//             finished panel E, so every other column becomes A[:, J] + E A[pivot rows, J] (pivot
+//             rows: E A[pivot rows, J]), one rank-8 update on the FP64 tensor path by all warps.
+// Without the inverse only the columns right of the panel are updated (E of an unused row is
+// -A21 A11^{-1}, so the update is the Schur complement).  Rows are interchanged by index only:
+// rlog is a row's logical place.  The interchanges permute the columns of the in-place inverse;
+// they are undone on the way out.
+// What bounds it is the chain of panel steps (pivot search, reciprocal, row broadcast); the CTAs
+// of an SM (four at N = 50) overlap theirs with each other's updates.  The form that ran all N
+// steps on block barriers, two a step, took 286 us for 1024 matrices of N = 50 (242 us without the
+// inverse), this one 176 (114).  Factorising the next panel beside the update (one warp ahead of three)
+// took 190 (150): the other CTAs already fill those slots.
+// ---------------------------------------------------------------------------------------------
+constexpr int GB_THREADS = 128;
+
+__host__ __device__ inline int gb_pitch(int N) { return N | 1; }          // matrix row pitch
+__host__ __device__ inline int gb_bpitch(int N) { return (N + 7) / 8 * 8 + 2; }  // pivot-row copy
+inline size_t gb_smem(int N) {
+  return (size_t(N) * gb_pitch(N) + 8 * size_t(gb_bpitch(N))) * sizeof(c128);
+}
+
+template <bool INVERT>
+__global__ void __launch_bounds__(GB_THREADS, 4)
+    gj_block_kernel(const c128* __restrict__ A, long strideA, c128* Ainv, long strideInv,
+                    c128* __restrict__ ovlp, int N, c128 post_scale, c128 post_add) {
+  constexpr unsigned FULL = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int P = gb_pitch(N), PB = gb_bpitch(N);
+  c128* a = reinterpret_cast<c128*>(smem_raw);  // [N][P]
+  c128* bc = a + size_t(N) * P;                 // [8][PB] the panel's pivot rows
+  __shared__ c128 xrow[2][8];                   // pivot row of the panel, by step parity
+  __shared__ c128 piv_val[64];
+  __shared__ int perm[64], rlog[64], at[64], pos[64];
+  __shared__ int prow[8];                       // physical row of the panel's pivots
+  __shared__ unsigned long long s_pivmask;      // ... as a bit mask
+  __shared__ int s_singular;
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const long w = blockIdx.x;
+  const c128* Aw = A + w * strideA;
+  for (int e = tid; e < N * N; e += GB_THREADS) {
+    const int i = e / N, j = e - i * N;
+    a[i * P + j] = Aw[e];
+  }
+  const int r0 = lane, r1 = lane + 32;  // warp 0: this lane's rows
+  const bool ok0 = r0 < N, ok1 = r1 < N;
+  int l0 = r0, l1 = r1;                 // their logical places
+  bool singular = false;
+  __syncthreads();
+
+  for (int k0 = 0; k0 < N; k0 += 8) {
+    const int nb = N - k0 < 8 ? N - k0 : 8;
+    c128 p0[8], p1[8];
+    unsigned long long pivmask = 0ull;
+    if (warp == 0) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        p0[c] = (ok0 && c < nb) ? a[r0 * P + k0 + c] : cmk(0.0, 0.0);
+        p1[c] = (ok1 && c < nb) ? a[r1 * P + k0 + c] : cmk(0.0, 0.0);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (j < nb) {
+          const int k = k0 + j;
+          // first max |re|+|im| of column k over the logical rows k..N-1 (NaN counts as 0)
+          const c128 f0 = p0[j], f1 = p1[j];
+          const bool c0 = ok0 && l0 >= k, c1 = ok1 && l1 >= k;
+          const double v0 = c0 ? cabs1(f0) : 0.0, v1 = c1 ? cabs1(f1) : 0.0;
+          const unsigned long long k0_ = (v0 == v0) ? static_cast<unsigned long long>(__double_as_longlong(v0)) : 0ull;
+          const unsigned long long k1_ = (v1 == v1) ? static_cast<unsigned long long>(__double_as_longlong(v1)) : 0ull;
+          const unsigned long long kl = k1_ > k0_ ? k1_ : k0_;
+          const unsigned mhi = __reduce_max_sync(FULL, unsigned(kl >> 32));
+          const unsigned mlo = __reduce_max_sync(FULL, unsigned(kl >> 32) == mhi ? unsigned(kl) : 0u);
+          const unsigned long long km = (static_cast<unsigned long long>(mhi) << 32) | mlo;
+          const unsigned i0 = (c0 && k0_ == km) ? unsigned(l0) * 64u + unsigned(r0) : FULL;
+          const unsigned i1 = (c1 && k1_ == km) ? unsigned(l1) * 64u + unsigned(r1) : FULL;
+          const unsigned id = __reduce_min_sync(FULL, i0 < i1 ? i0 : i1);
+          const int p = int(id >> 6), pr = int(id & 63u);  // logical place and row of the pivot
+          const bool zero = km == 0ull;
+          const bool m0 = pr == r0, m1 = pr == r1;
+          if (m0 || m1) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) xrow[j & 1][c] = m0 ? p0[c] : p1[c];
+          }
+          __syncwarp();
+          const c128 piv = xrow[j & 1][j];
+          const double rden = 1.0 / (piv.x * piv.x + piv.y * piv.y);
+          const c128 dinv = cmk(piv.x * rden, -piv.y * rden);
+          // logical rows after the interchange
+          if (m0) l0 = k; else if (l0 == k) l0 = p;
+          if (m1) l1 = k; else if (l1 == k) l1 = p;
+          if (lane == 0) {
+            piv_val[k] = piv;
+            perm[k] = p;
+            prow[j] = pr;
+          }
+          pivmask |= 1ull << pr;
+          singular = singular || zero;
+          const c128 g0 = cmul(f0, dinv), g1 = cmul(f1, dinv);
+          const bool u0 = !zero && !m0 && (INVERT || l0 > k), u1 = !zero && !m1 && (INVERT || l1 > k);
+          const bool s0 = !zero && m0 && INVERT, s1 = !zero && m1 && INVERT;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            if (c == j) continue;
+            const c128 x = xrow[j & 1][c];
+            if (u0) {
+              p0[c].x = fma(-g0.x, x.x, fma(g0.y, x.y, p0[c].x));
+              p0[c].y = fma(-g0.x, x.y, fma(-g0.y, x.x, p0[c].y));
+            } else if (s0) {
+              p0[c] = cmul(x, dinv);
+            }
+            if (u1) {
+              p1[c].x = fma(-g1.x, x.x, fma(g1.y, x.y, p1[c].x));
+              p1[c].y = fma(-g1.x, x.y, fma(-g1.y, x.x, p1[c].y));
+            } else if (s1) {
+              p1[c] = cmul(x, dinv);
+            }
+          }
+          p0[j] = u0 ? cmk(-g0.x, -g0.y) : (s0 ? dinv : cmk(0.0, 0.0));
+          p1[j] = u1 ? cmk(-g1.x, -g1.y) : (s1 ? dinv : cmk(0.0, 0.0));
+        }
+      }
+      if (lane == 0) s_pivmask = pivmask;
+    }
+    __syncthreads();
+    // warp 0 stores the finished panel; the others copy the pivot rows' other columns
+    const int j_lo = INVERT ? 0 : k0 + 8;
+    if (warp == 0) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (c < nb) {
+          // without the inverse a used row takes no further part: its multipliers are zero
+          if (ok0) a[r0 * P + k0 + c] = (INVERT || l0 >= k0 + nb) ? p0[c] : cmk(0.0, 0.0);
+          if (ok1) a[r1 * P + k0 + c] = (INVERT || l1 >= k0 + nb) ? p1[c] : cmk(0.0, 0.0);
+        }
+    } else {
+      for (int q = warp - 1; q < 8; q += GB_THREADS / 32 - 1)
+        for (int j = j_lo + lane; j < PB - 2; j += 32)
+          if (j < k0 || j >= k0 + 8)
+            bc[q * PB + j] = (q < nb && j < N) ? a[prow[q] * P + j] : cmk(0.0, 0.0);
+    }
+    __syncthreads();
+    const unsigned long long pm = s_pivmask;
+    const int nt = (N + 7) / 8, kt = k0 / 8;
+    for (int e = warp; e < nt * nt; e += GB_THREADS / 32) {
+      const int tc = e / nt, tr = e - tc * nt;
+      if (tc == kt || (!INVERT && tc < kt)) continue;
+      const int row = tr * 8 + g, col = tc * 8 + 2 * t;
+      const bool rok = row < N, keep = rok && !((pm >> row) & 1ull);
+      c128* ar = a + (rok ? row : 0) * P;
+      double cr[2] = {0.0, 0.0}, ci[2] = {0.0, 0.0};
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (keep && col + h < N) {
+          const c128 v = ar[col + h];
+          cr[h] = v.x;
+          ci[h] = v.y;
+        }
+#pragma unroll
+      for (int kk = 0; kk < 8; kk += 4) {
+        const c128 fa = (rok && kk + t < nb) ? ar[k0 + kk + t] : cmk(0.0, 0.0);
+        const c128 fb = bc[(kk + t) * PB + tc * 8 + g];
+        zmma(cr, ci, fa, fb);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (rok && col + h < N && (INVERT || keep)) ar[col + h] = cmk(cr[h], ci[h]);
+    }
+    __syncthreads();
+  }
+
+  if (warp == 0) {
+    if (ok0) rlog[r0] = l0;
+    if (ok1) rlog[r1] = l1;
+    if (lane == 0) s_singular = singular ? 1 : 0;
+    double sr = 0.0, si = 0.0;
+    for (int k = lane; k < N; k += 32) {
+      const c128 l = log_pivot(piv_val[k], perm[k] != k);
+      sr += l.x;
+      si += l.y;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      sr += __shfl_xor_sync(FULL, sr, off);
+      si += __shfl_xor_sync(FULL, si, off);
+    }
+    if (lane == 0)
+      ovlp[w] = cadd(cmul(post_scale, wrap_imag(cadd(ovlp[w], cmk(sr, si)))), post_add);
+  }
+  if (INVERT) {
+    // at[c] = column of the in-place result that ends in column c; pos is its inverse
+    if (tid < N) at[tid] = tid;
+    __syncthreads();
+    if (tid == 0)
+      for (int k = N - 1; k >= 0; --k) {
+        const int q = perm[k], x = at[k];
+        at[k] = at[q];
+        at[q] = x;
+      }
+    __syncthreads();
+    if (tid < N) pos[at[tid]] = tid;
+    __syncthreads();
+    c128* Iw = Ainv + w * strideInv;
+    const bool sing = s_singular != 0;
+    for (int e = tid; e < N * N; e += GB_THREADS) {
+      const int i = e / N, j = e - i * N;
+      Iw[long(rlog[i]) * N + pos[j]] = sing ? cmk(0.0, 0.0) : a[i * P + j];
+    }
+  }
+}
+
 int batched_logdet_inverse(cudaStream_t s, const c128* A, long strideA, c128* Ainv, long strideInv,
                            c128* ovlp, int W, int N, bool invert, c128 post_scale, c128 post_add) {
   if (W <= 0 || N <= 0) return AFQMC_OK;
   if (N <= 64) {
-    if (N <= 8)
-      launch_gj_reg<4, 2>(s, A, strideA, Ainv, strideInv, ovlp, W, N, invert, post_scale, post_add);
-    else if (N <= 16)
-      launch_gj_reg<8, 2>(s, A, strideA, Ainv, strideInv, ovlp, W, N, invert, post_scale, post_add);
-    else if (N <= 32)
+#define GJ_WARP(G, NC)   \
+  if (N <= NC) {         \
+    launch_gj_warp<G, NC>(s, A, strideA, Ainv, strideInv, ovlp, W, N, invert, post_scale, post_add); \
+    return launch_status("gj_warp_kernel"); \
+  }
+    GJ_WARP(4, 4) GJ_WARP(8, 8) GJ_WARP(16, 12) GJ_WARP(16, 16)
+#undef GJ_WARP
+    if (N <= 32) {
       launch_gj_reg<16, 2>(s, A, strideA, Ainv, strideInv, ovlp, W, N, invert, post_scale,
                            post_add);
-    else if (N <= 52)
-      launch_gj_reg<13, 4>(s, A, strideA, Ainv, strideInv, ovlp, W, N, invert, post_scale,
-                           post_add);
-    else
-      launch_gj_reg<16, 4>(s, A, strideA, Ainv, strideInv, ovlp, W, N, invert, post_scale,
-                           post_add);
-    return launch_status("gj_reg_kernel");
+      return launch_status("gj_reg_kernel");
+    }
+    const size_t smem = gb_smem(N);
+    if (invert) {
+      AFQMC_CUDA_TRY(cudaFuncSetAttribute(gj_block_kernel<true>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      gj_block_kernel<true><<<W, GB_THREADS, smem, s>>>(A, strideA, Ainv, strideInv, ovlp, N,
+                                                        post_scale, post_add);
+    } else {
+      AFQMC_CUDA_TRY(cudaFuncSetAttribute(gj_block_kernel<false>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      gj_block_kernel<false><<<W, GB_THREADS, smem, s>>>(A, strideA, nullptr, 0, ovlp, N,
+                                                         post_scale, post_add);
+    }
+    return launch_status("gj_block_kernel");
   }
   const int P = invert ? 2 * N : N;
   const int PP = P | 1;

@@ -13,10 +13,16 @@
 // (complex) and 8-byte (real) elements.  With few output tiles, a cluster of `split` CTAs along z
 // shares one tile's K range and adds the partial sums through distributed shared memory in rank
 // order.
+//
+// Rates at 1024 walkers, of 35.5 TFLOP/s (cuBLAS DGEMM): 28.8 for the vHS pairs (K = 1600), 26.6
+// for vbias (K = 10000; 400 tiles on 148 SMs leave a tenth idle), 24.2 for the Taylor product
+// (200 x 50 x 200, padded to 224 x 56).  With 64 x 64 tiles throughout, and register staging in
+// place of cp.async, the last ran at 16.
 #pragma once
 
 #include <cooperative_groups.h>
 
+#include "dmma.cuh"
 #include "zgemm.cuh"
 
 namespace afqmc {
@@ -25,12 +31,6 @@ namespace zg {
 constexpr int BK = 16;
 constexpr int STAGES = 3;
 constexpr int MAX_WARPS = 8;
-
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
 
 // one element from global to shared memory, zero when `in` is false (the address is not read)
 __device__ __forceinline__ void copy_async(c128* dst, const c128* src, bool in) {
@@ -286,8 +286,9 @@ int launch(cudaStream_t s, int batch, const GemmParams& p, const Shape& sh) {
   const int bm = 8 * sh.warps, bn = 8 * TN;
   size_t smem = size_t(STAGES) * O::stage_bytes(bm, bn);
   if (sh.split > 1 && smem < size_t(bm) * bn * sizeof(c128)) smem = size_t(bm) * bn * sizeof(c128);
-  AFQMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(smem)));
+  if (smem > 48 * 1024)
+    AFQMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        int(smem)));
   unsigned gx = ceil_div(p.n, bn);
   if (SYM) {
     const unsigned nb = ceil_div(p.sym_m, 8);

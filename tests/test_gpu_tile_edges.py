@@ -12,6 +12,32 @@ pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -53
 
 
+@pytest.mark.parametrize("N", [1, 3, 4, 5, 8, 9, 12, 13, 16, 17, 20, 21, 24, 28, 29, 32, 33, 40, 41,
+                               50, 57, 63, 64, 65])
+@pytest.mark.parametrize("W", [1, 37])
+def test_inverse_logdet(cuda, N, W):
+    from safire_b200 import afqmc as A
+    rs = np.random.default_rng(N)
+    a = rand_c(rs, W, N, N)
+    a[:, np.arange(N), np.arange(N)] *= 1e-3  # pivoting matters
+    if N > 1:
+        a[W - 1, :, N - 1] = a[W - 1, :, 0]   # singular to rounding: checked apart
+    d_inv = torch.zeros((W, N, N), dtype=torch.complex128, device=cuda)
+    d_log = torch.zeros(W, dtype=torch.complex128, device=cuda)
+    A.det_ops.inverse_logdet(to_dev(a), d_inv, d_log)
+    inv, log = to_host(d_inv), to_host(d_log)
+    for w in range(W if N == 1 else W - 1):
+        cond = np.linalg.cond(a[w])
+        assert np.linalg.norm(inv[w] @ a[w] - np.eye(N), 2) < 50 * N * EPS * cond
+        sign, la = np.linalg.slogdet(a[w])
+        assert abs(log[w].real - la) < 50 * N * EPS * cond
+        assert abs(np.exp(1j * log[w].imag) - sign) < 50 * N * EPS * cond
+    # a zero column is singular exactly: a zero inverse
+    a[:, :, 0] = 0.0
+    A.det_ops.inverse_logdet(to_dev(a), d_inv, d_log)
+    assert np.all(to_host(d_inv) == 0)
+
+
 def _ham(M, N, Nc, L):
     from safire_b200 import afqmc as A
     _, orb = np.linalg.eigh(np.diag(np.arange(M, dtype=float)) + 0.1)
