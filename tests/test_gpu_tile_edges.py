@@ -38,6 +38,25 @@ def test_inverse_logdet(cuda, N, W):
     assert np.all(to_host(d_inv) == 0)
 
 
+@pytest.mark.parametrize("M,N", [(9, 1), (8, 8), (30, 9), (40, 31), (64, 32), (70, 50), (80, 64),
+                                 (101, 83)])
+def test_orthogonalize(cuda, M, N):
+    from safire_b200 import afqmc as A
+    rs = np.random.default_rng(M)
+    W = 5
+    S = np.eye(M, N) + rand_c(rs, W, M, N, scale=0.3 / np.sqrt(M))
+    d, ld = to_dev(S), torch.zeros(W, dtype=torch.complex128, device=cuda)
+    A.det_ops.orthogonalize(d, ld)
+    Q, ld = to_host(d), to_host(ld)
+    for w in range(W):
+        q, r = np.linalg.qr(S[w])
+        ph = np.diag(r) / np.abs(np.diag(r))
+        tol = 50 * N * EPS * np.linalg.cond(S[w])
+        assert np.linalg.norm(Q[w].conj().T @ Q[w] - np.eye(N), 2) < 50 * N * EPS
+        assert np.max(np.abs(Q[w] - q * ph)) < tol
+        assert abs(ld[w] - np.sum(np.log(np.abs(np.diag(r))))) < tol
+
+
 def _ham(M, N, Nc, L):
     from safire_b200 import afqmc as A
     _, orb = np.linalg.eigh(np.diag(np.arange(M, dtype=float)) + 0.1)
