@@ -57,6 +57,30 @@ def test_orthogonalize(cuda, M, N):
         assert abs(ld[w] - np.sum(np.log(np.abs(np.diag(r))))) < tol
 
 
+@pytest.mark.parametrize("M,N", [(5, 1), (19, 3), (32, 8), (32, 32), (33, 9), (64, 16), (65, 24),
+                                 (101, 23), (128, 32), (129, 8), (70, 33)])
+@pytest.mark.parametrize("order", [0, 1, 6])
+def test_propagate(cuda, M, N, order):
+    from safire_b200 import afqmc as A
+    rs = np.random.default_rng(M + N)
+    W = 3
+    P1 = np.eye(M) + rand_c(rs, M, M, scale=0.1 / np.sqrt(M))
+    V = rand_c(rs, W, M, M, scale=0.5 / np.sqrt(M))
+    S = rand_c(rs, W, M, N)
+    d = torch.zeros((W, M * N + 3), dtype=torch.complex128, device=cuda)  # a longer walker row
+    view = d[:, :M * N].unflatten(1, (M, N))
+    view.copy_(to_dev(S))
+    A.det_ops.Propagate(view, to_dev(P1), to_dev(V), order)
+    T = P1 @ S
+    R = T.copy()
+    for n in range(1, order + 1):
+        T = (1j / n) * (V @ T)
+        R = R + T
+    want = P1 @ R
+    assert np.max(np.abs(to_host(view) - want)) < 50 * M * EPS * np.max(np.abs(want))
+    assert torch.all(d[:, M * N:] == 0)
+
+
 def _ham(M, N, Nc, L):
     from safire_b200 import afqmc as A
     _, orb = np.linalg.eigh(np.diag(np.arange(M, dtype=float)) + 0.1)
