@@ -496,14 +496,23 @@ EnergyArgs energy_args(afqmc_ham_s* h, const c128* G, long ldG) {
   return a;
 }
 
-// exchange-tensor chunk budget (complex elements): 256 MiB, at least one walker
-long energy_chunk_elems(afqmc_ham_s* h, int W) {
+// Exchange-tensor chunk (complex elements): 256 MiB, at least one walker.  *rows receives the
+// elements that a chunk's gathered G rows take, for the spin blocks whose rows are not contiguous.
+long energy_chunk_elems(afqmc_ham_s* h, int W, long ldG, long* rows) {
   int nmax = h->nel[0] > h->nel[1] ? h->nel[0] : h->nel[1];
   long per = long(nmax) * h->Nc * nmax;
   long budget = (256l << 20) / long(sizeof(c128));
   long nw = budget / (per > 0 ? per : 1);
   if (nw < 1) nw = 1;
   if (nw > W) nw = W;
+  *rows = 0;
+  for (int sp = 0; sp < h->nspin; ++sp) {
+    const long n = h->nel[sp];
+    if (n == 0 || ldG == n * h->M) continue;
+    // a spin block fits as many of its walkers as its own T allows
+    const long wc = std::min<long>(W, nw * per / (n * h->Nc * n));
+    *rows = std::max(*rows, wc * n * h->M);
+  }
   return nw * per;
 }
 
@@ -529,8 +538,9 @@ int ham_energy(afqmc_ham_s* h, cudaStream_t s, const c128* G, long ldG, c128* E,
   bool fused = tc != nullptr;
   for (int sp = 0; sp < h->nspin && fused; ++sp)
     if (h->nel[sp] > 0 && !exchange_fused_ok(tc, sp)) fused = false;
-  const long chunk = fused ? 0 : energy_chunk_elems(h, W);
-  if (!fused) AFQMC_TRY(wT.get(sizeof(c128) * size_t(chunk), s));
+  long rows = 0;
+  const long chunk = fused ? 0 : energy_chunk_elems(h, W, ldG, &rows);
+  if (!fused) AFQMC_TRY(wT.get(sizeof(c128) * size_t(chunk + rows), s));
   AFQMC_TRY(ex.get(sizeof(c128) * size_t(W) * h->Nc, s));
   AFQMC_TRY(kl.get(sizeof(c128) * size_t(W) * h->Nc, s));
   return energy_fp64(s, a, E, W, addH1, addEJ, addEXX, (c128*)wT.p, chunk, (c128*)ex.p,

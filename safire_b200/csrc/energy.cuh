@@ -23,7 +23,9 @@ struct EnergyArgs {
 
 struct MixedHam;
 
-// complex128 path (and mixed-precision exchange GEMM when tc is given).  workT: chunk workspace of workT_elems complex elements; exx_part, Kl: [W][Nc].
+// complex128 path (and mixed-precision exchange GEMM when tc is given).  workT: chunk workspace of
+// workT_elems complex elements, and behind them a chunk's G rows of one spin block where a walker's
+// row holds more than that block; exx_part, Kl: [W][Nc].
 // tc != nullptr: the exchange tensor chunks come from the tensor-core GEMM (mixed precision).
 int energy_fp64(cudaStream_t s, const EnergyArgs& a, c128* E, int W, bool addH1, bool addEJ,
                 bool addEXX, c128* workT, long workT_elems, c128* exx_part, c128* Kl,
