@@ -41,6 +41,13 @@ __device__ __forceinline__ c64 csub(c64 a, c64 b) { return make_float2(a.x - b.x
 __device__ __forceinline__ c64 cmul(c64 a, c64 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+// o + a b as four chained multiply-adds (cadd of a cmul takes six operations)
+__device__ __forceinline__ c64 cfma(c64 a, c64 b, c64 o) {
+  return make_float2(fmaf(-a.y, b.y, fmaf(a.x, b.x, o.x)), fmaf(a.y, b.x, fmaf(a.x, b.y, o.y)));
+}
+__device__ __forceinline__ c128 cfma(c128 a, c128 b, c128 o) {
+  return cmk(fma(-a.y, b.y, fma(a.x, b.x, o.x)), fma(a.y, b.x, fma(a.x, b.y, o.y)));
+}
 __device__ __forceinline__ c64 cscale(c64 a, float s) { return make_float2(a.x * s, a.y * s); }
 template <typename R> struct CxOf;
 template <> struct CxOf<double> { using T = c128; };
@@ -233,24 +240,59 @@ __global__ void gather_ref_rows_kernel(const c128* __restrict__ TMN, const int* 
   }
 }
 
-// ov[w][u] = det(QQ0[w][particles_u][holes_u]) for every unique excitation u >= 1 (ov[w][0] = 1):
-// partial-pivoting LU of the nex x nex block in registers / local memory (nex <= PH_NEX_MAX).
-__global__ void excitation_det_kernel(const c128* __restrict__ QQ0, const int* __restrict__ uoff,
-                                      const int* __restrict__ unex, const int* __restrict__ uexc,
-                                      int nuniq, int W, int nact, int N, c128* __restrict__ ov) {
-  const long t = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= long(nuniq) * W) return;
-  const int w = int(t / nuniq), u = int(t - long(w) * nuniq);
-  if (u == 0) {
-    ov[t] = cmk(1.0, 0.0);
-    return;
+// Determinant of the N x N excitation block a[p][q] = QQ0[particle_p][hole_q] (e = holes then
+// particles) by partial-pivoting LU, in registers (row interchanges by selects).
+template <int N>
+__device__ __forceinline__ c128 excitation_det(const c128* __restrict__ Q, const int* __restrict__ e,
+                                               int nel) {
+  c128 a[N][N];
+#pragma unroll
+  for (int p = 0; p < N; ++p)
+#pragma unroll
+    for (int q = 0; q < N; ++q) a[p][q] = Q[size_t(e[N + p]) * nel + e[q]];
+  c128 det = cmk(1.0, 0.0);
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    int piv = k;
+    double best = cabs1(a[k][k]);
+#pragma unroll
+    for (int i = k + 1; i < N; ++i) {
+      const double v = cabs1(a[i][k]);
+      if (v > best) {
+        best = v;
+        piv = i;
+      }
+    }
+    if (!(best > 0.0)) return cmk(0.0, 0.0);
+#pragma unroll
+    for (int i = k + 1; i < N; ++i)
+      if (piv == i) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          const c128 x = a[k][j];
+          a[k][j] = a[i][j];
+          a[i][j] = x;
+        }
+      }
+    if (piv != k) det = cmk(-det.x, -det.y);
+    det = cmul(det, a[k][k]);
+    const c128 dinv = cdiv(cmk(1.0, 0.0), a[k][k]);
+#pragma unroll
+    for (int i = k + 1; i < N; ++i) {
+      const c128 f = cmul(a[i][k], dinv);
+#pragma unroll
+      for (int j = k + 1; j < N; ++j) a[i][j] = csub(a[i][j], cmul(f, a[k][j]));
+    }
   }
-  const int n = unex[u];
-  const int* e = uexc + uoff[u];
-  const c128* Q = QQ0 + size_t(w) * nact * N;
+  return det;
+}
+
+// the same for any n <= PH_NEX_MAX, in local memory
+__device__ __noinline__ c128 excitation_det_any(const c128* __restrict__ Q,
+                                                const int* __restrict__ e, int n, int nel) {
   c128 a[PH_NEX_MAX][PH_NEX_MAX];
   for (int p = 0; p < n; ++p)
-    for (int q = 0; q < n; ++q) a[p][q] = Q[size_t(e[n + p]) * N + e[q]];
+    for (int q = 0; q < n; ++q) a[p][q] = Q[size_t(e[n + p]) * nel + e[q]];
   c128 det = cmk(1.0, 0.0);
   for (int k = 0; k < n; ++k) {
     int piv = k;
@@ -262,10 +304,7 @@ __global__ void excitation_det_kernel(const c128* __restrict__ QQ0, const int* _
         piv = i;
       }
     }
-    if (!(best > 0.0)) {
-      det = cmk(0.0, 0.0);
-      break;
-    }
+    if (!(best > 0.0)) return cmk(0.0, 0.0);
     if (piv != k) {
       for (int j = 0; j < n; ++j) {
         const c128 x = a[k][j];
@@ -281,7 +320,30 @@ __global__ void excitation_det_kernel(const c128* __restrict__ QQ0, const int* _
       for (int j = k + 1; j < n; ++j) a[i][j] = csub(a[i][j], cmul(f, a[k][j]));
     }
   }
-  ov[t] = det;
+  return det;
+}
+
+// ov[w][u] = det(QQ0[w][particles_u][holes_u]) for every unique excitation u >= 1 (ov[w][0] = 1)
+__global__ void excitation_det_kernel(const c128* __restrict__ QQ0, const int* __restrict__ uoff,
+                                      const int* __restrict__ unex, const int* __restrict__ uexc,
+                                      int nuniq, int W, int nact, int N, c128* __restrict__ ov) {
+  const long t = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= long(nuniq) * W) return;
+  const int w = int(t / nuniq), u = int(t - long(w) * nuniq);
+  if (u == 0) {
+    ov[t] = cmk(1.0, 0.0);
+    return;
+  }
+  const int n = unex[u];
+  const int* e = uexc + uoff[u];
+  const c128* Q = QQ0 + size_t(w) * nact * N;
+  switch (n) {
+    case 1: ov[t] = excitation_det<1>(Q, e, N); break;
+    case 2: ov[t] = excitation_det<2>(Q, e, N); break;
+    case 3: ov[t] = excitation_det<3>(Q, e, N); break;
+    case 4: ov[t] = excitation_det<4>(Q, e, N); break;
+    default: ov[t] = excitation_det_any(Q, e, n, N); break;
+  }
 }
 
 // ovlp[w] = log(sum_k c_k ov_up[w][det_up k] ov_dn[w][det_dn k]) + logov[w]  (PHMSD.cpp:884-896)
@@ -475,8 +537,80 @@ __global__ void compact_R_kernel(const c128* __restrict__ QQ0, const int* __rest
   }
 }
 
+// The same for a compile-time size, in registers (row interchanges by selects).
+template <int N>
+__device__ __forceinline__ bool block_inverse(const c128* __restrict__ Q0, const int* __restrict__ e,
+                                              int nel, c128 (&inv)[N][N]) {
+  c128 a[N][N];
+#pragma unroll
+  for (int p = 0; p < N; ++p)
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      a[p][q] = Q0[size_t(e[N + p]) * nel + e[q]];
+      inv[p][q] = cmk(p == q ? 1.0 : 0.0, 0.0);
+    }
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    int piv = k;
+    double best = cabs1(a[k][k]);
+#pragma unroll
+    for (int i = k + 1; i < N; ++i)
+      if (cabs1(a[i][k]) > best) {
+        best = cabs1(a[i][k]);
+        piv = i;
+      }
+    if (!(best > 0.0)) return false;
+#pragma unroll
+    for (int i = k + 1; i < N; ++i)
+      if (piv == i) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          c128 x = a[k][j]; a[k][j] = a[i][j]; a[i][j] = x;
+          x = inv[k][j]; inv[k][j] = inv[i][j]; inv[i][j] = x;
+        }
+      }
+    const c128 dinv = cdiv(cmk(1.0, 0.0), a[k][k]);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      a[k][j] = cmul(a[k][j], dinv);
+      inv[k][j] = cmul(inv[k][j], dinv);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (i != k) {
+        const c128 f = a[i][k];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          a[i][j] = csub(a[i][j], cmul(f, a[k][j]));
+          inv[i][j] = csub(inv[i][j], cmul(f, inv[k][j]));
+        }
+      }
+  }
+  return true;
+}
+
+// inverse of one excitation block to o (row-major) and, if given, in complex64 to o32 with the
+// stride es; zeros for a singular block
+template <int N>
+__device__ __forceinline__ void store_block_inverse(const c128* __restrict__ Q0,
+                                                    const int* __restrict__ e, int nel,
+                                                    c128* __restrict__ o, float2* __restrict__ o32,
+                                                    int es) {
+  c128 inv[N][N];
+  const bool ok = block_inverse<N>(Q0, e, nel, inv);
+#pragma unroll
+  for (int p = 0; p < N; ++p)
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      const c128 v = ok ? inv[p][q] : cmk(0.0, 0.0);
+      o[p * N + q] = v;
+      if (o32) o32[size_t(p * N + q) * es] = make_float2(float(v.x), float(v.y));
+    }
+}
+
 // INV[w][uinv[u] ...] = inverse of the excitation block of every unique excitation u >= 1
 // (row-major nex x nex), zeros for a singular block: the Q matrices of the Woodbury R.
+// INV32: the same in complex64, structure-of-arrays within the shell (entry k at base + k cnt).
 __global__ void woodbury_inverses_kernel(const c128* __restrict__ QQ0, const int* __restrict__ uoff,
                                          const int* __restrict__ unex,
                                          const int* __restrict__ uexc,
@@ -488,19 +622,31 @@ __global__ void woodbury_inverses_kernel(const c128* __restrict__ QQ0, const int
   if (t >= long(nuniq - 1) * W) return;
   const int w = int(t / (nuniq - 1)), u = 1 + int(t - long(w) * (nuniq - 1));
   const int nex = unex[u];
-  c128 inv[PH_NEX_MAX][PH_NEX_MAX];
-  const bool ok = woodbury_block_inverse(QQ0 + size_t(w) * nact * nel, uexc + uoff[u], nex, nel,
-                                         inv);
+  const int* e = uexc + uoff[u];
+  const c128* Q0 = QQ0 + size_t(w) * nact * nel;
   c128* o = INV + size_t(w) * ninv + uinv[u];
-  for (int p = 0; p < nex; ++p)
-    for (int q = 0; q < nex; ++q) o[p * nex + q] = ok ? inv[p][q] : cmk(0.0, 0.0);
-  if (INV32) {  // structure-of-arrays within the shell: entry k at base + k cnt
+  float2* o32 = nullptr;
+  int es = 0;
+  if (INV32) {
     const int4 hs = uhdrs[u];
-    float2* o32 = INV32 + size_t(w) * ninv + hs.z;
-    for (int p = 0; p < nex; ++p)
-      for (int q = 0; q < nex; ++q)
-        o32[size_t(p * nex + q) * hs.w] = ok ? make_float2(float(inv[p][q].x), float(inv[p][q].y))
-                                             : make_float2(0.f, 0.f);
+    o32 = INV32 + size_t(w) * ninv + hs.z;
+    es = hs.w;
+  }
+  switch (nex) {
+    case 1: store_block_inverse<1>(Q0, e, nel, o, o32, es); break;
+    case 2: store_block_inverse<2>(Q0, e, nel, o, o32, es); break;
+    case 3: store_block_inverse<3>(Q0, e, nel, o, o32, es); break;
+    case 4: store_block_inverse<4>(Q0, e, nel, o, o32, es); break;
+    default: {
+      c128 inv[PH_NEX_MAX][PH_NEX_MAX];
+      const bool ok = woodbury_block_inverse(Q0, e, nex, nel, inv);
+      for (int p = 0; p < nex; ++p)
+        for (int q = 0; q < nex; ++q) {
+          const c128 v = ok ? inv[p][q] : cmk(0.0, 0.0);
+          o[p * nex + q] = v;
+          if (o32) o32[size_t(p * nex + q) * es] = make_float2(float(v.x), float(v.y));
+        }
+    }
   }
 }
 
@@ -985,14 +1131,19 @@ __global__ void finish_energy_kernel(const c128* __restrict__ Ov, const c128* __
 // The last term is summed as A QQ0 (A[h][b] = sum of c over (u, a, q) with h_a = h, p_q = b) onto
 // the reference orbitals r_i, and the hole electrons' share is moved from r_{h_e} to p_e per
 // determinant.  Every electron row also gets sum_u wu at r_i (the identity of every determinant).
-// Shared-memory atomics order the sums differently from run to run (the reference reduces R with
-// atomics too).
+//
+// Each row h belongs to a group of eight lanes, which walks the list of the (u, a) with h_a = h
+// (hrow, hent = {nex | a << 8, offset in uexc, offset in INV, u}) in order: lane l takes hole and
+// particle l of the determinant, all different, so its additions to the row need no atomics
+// and the sums have one order.  (With a thread per determinant and double-precision atomics in
+// shared memory, which are compare-and-swap loops meeting on the reference columns, 512 walkers
+// of 50 determinants took 43 us a spin; 1536 take 51 here.)  The next entry's data are fetched ahead.
 constexpr int PHR_THREADS = 256;
 __global__ void __launch_bounds__(PHR_THREADS) phmsd_R_kernel(
-    const c128* __restrict__ QQ0, const int* __restrict__ refc, const int* __restrict__ uoff,
-    const int* __restrict__ unex, const int* __restrict__ uexc, const int* __restrict__ uinv,
-    const c128* __restrict__ INV, int ninv, const c128* __restrict__ wgt, int nuniq, int W,
-    int nel, int nact, c128* __restrict__ R) {
+    const c128* __restrict__ QQ0, const int* __restrict__ refc, const int* __restrict__ hrow,
+    const int4* __restrict__ hent, const int* __restrict__ uexc, const c128* __restrict__ INV,
+    int ninv, const c128* __restrict__ wgt, int nuniq, int W, int nel, int nact,
+    c128* __restrict__ R) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int NA = nel * nact;
   c128* Rs = reinterpret_cast<c128*>(smem_raw);  // [nel][nact]
@@ -1012,36 +1163,48 @@ __global__ void __launch_bounds__(PHR_THREADS) phmsd_R_kernel(
   block_sum3(ws, z1, z2, red);
   if (threadIdx.x == 0) wsum = ws;
   __syncthreads();
-  auto add = [](c128* x, c128 v) {
-    atomicAdd(&x->x, v.x);
-    atomicAdd(&x->y, v.y);
-  };
   const c128* Iw = INV + size_t(w) * ninv;
-  for (int u = 1 + threadIdx.x; u < nuniq; u += blockDim.x) {
-    const c128 wu = wgt[size_t(u) * W + w];
-    if (wu.x == 0.0 && wu.y == 0.0) continue;
-    const int nex = unex[u];
-    const int* e = uexc + uoff[u];
-    const c128* Qi = Iw + uinv[u];
-    for (int a = 0; a < nex; ++a) {
-      const int ha = e[a], pa = e[nex + a];
-      c128* Ra = Rs + ha * nact;
-      c128* Aa = As + ha * nact;
-      add(Ra + pa, wu);
-      add(Ra + refc[ha], cmk(-wu.x, -wu.y));
-      for (int q = 0; q < nex; ++q) {
-        const c128 c = cmul(wu, Qi[a * nex + q]);
-        add(Ra + e[nex + q], c);
-        add(Aa + e[nex + q], c);
+  const int l = threadIdx.x & 7;
+  const unsigned mask = 0xffu << (threadIdx.x & 24);  // this group's lanes
+  for (int h = threadIdx.x >> 3; h < nel; h += blockDim.x >> 3) {
+    c128* Rh = Rs + h * nact;
+    c128* Ah = As + h * nact;
+    const int e0 = hrow[h], e1 = hrow[h + 1];
+    // an entry's weight, this lane's hole, particle and element of Q's row a
+    int4 en = make_int4(0, 0, 0, 0);
+    c128 wu = cmk(0, 0), q = cmk(0, 0);
+    int hx = 0, px = 0;
+    auto fetch = [&](int e) {
+      en = hent[e];
+      const int n = en.x & 255, a = en.x >> 8;
+      wu = wgt[size_t(en.w) * W + w];
+      if (l < n) {
+        hx = uexc[en.y + l];
+        px = uexc[en.y + n + l];
+        q = Iw[en.z + a * n + l];
       }
-      for (int x = 0; x < nex; ++x) {
-        const int hx = e[x];
-        c128 sx = cmk(0, 0);
-        for (int q = 0; q < nex; ++q)
-          sx = cadd(sx, cmul(cmul(wu, Qi[a * nex + q]), Qs[e[nex + q] * nel + hx]));
-        add(Ra + refc[hx], sx);
-        add(Ra + e[nex + x], cmk(-sx.x, -sx.y));
+    };
+    if (e0 < e1) fetch(e0);
+    for (int e = e0; e < e1; ++e) {
+      const int n = en.x & 255, a = en.x >> 8, ph = hx, pp = px;
+      const c128 wc = wu, c = cmul(wu, q);
+      if (e + 1 < e1) fetch(e + 1);
+      c128 sx = cmk(0, 0);
+      for (int j = 0; j < n; ++j) {
+        const c128 cj = cmk(__shfl_sync(mask, c.x, j, 8), __shfl_sync(mask, c.y, j, 8));
+        const int pj = __shfl_sync(mask, pp, j, 8);
+        if (l < n) sx = cfma(cj, Qs[pj * nel + ph], sx);
       }
+      const bool use = l < n && (wc.x != 0.0 || wc.y != 0.0);
+      // what leaves the reference orbital comes to the particle
+      const c128 d = csub(l == a ? wc : cmk(0, 0), sx);
+      if (use) {
+        Rh[pp] = cadd(Rh[pp], cadd(c, d));
+        Ah[pp] = cadd(Ah[pp], c);
+      }
+      __syncwarp(mask);
+      if (use) Rh[refc[ph]] = csub(Rh[refc[ph]], d);
+      __syncwarp(mask);
     }
   }
   __syncthreads();
@@ -1185,6 +1348,9 @@ struct afqmc_phmsd_s {
   c128* Rfull = nullptr;
   // offset of every unique excitation's inverse block (nex^2 entries) and the total per walker
   int* uinv[2] = {nullptr, nullptr};
+  // per hole electron, the (excitation, position) pairs it is a hole of (phmsd_R_kernel)
+  int* hrow[2] = {nullptr, nullptr};
+  int4* hent[2] = {nullptr, nullptr};
   int ninv[2] = {0, 0};
   // energy tables: hole rows (electrons that are a hole of some excitation) and virtual columns
   // (active orbitals outside the reference); per excitation its holes, particles, hole rows and
@@ -1276,6 +1442,8 @@ struct afqmc_phmsd_s {
       cudaFree(rowptr[s]);
       cudaFree(kidx[s]);
       cudaFree(uinv[s]);
+      cudaFree(hrow[s]);
+      cudaFree(hent[s]);
       cudaFree(hl[s]);
       cudaFree(vl[s]);
       cudaFree(uexc4[s]);
@@ -1481,6 +1649,18 @@ extern "C" int afqmc_phmsd_create(int M, int nup, int ndn, int nact_up, int nact
       h->ninv[s] += nex[s][u] * nex[s][u];
     }
     AFQMC_TRY(to_device(&h->uinv[s], io.data(), io.size()));
+    std::vector<int> hp(size_t(nel[s]) + 1, 0);
+    for (int u = 1; u < nuniq[s]; ++u)
+      for (int a = 0; a < nex[s][u]; ++a) ++hp[excs[s][off[s][u] + a] + 1];
+    for (int i = 0; i < nel[s]; ++i) hp[i + 1] += hp[i];
+    std::vector<int> hpos(hp.begin(), hp.end() - 1);
+    std::vector<int4> he(size_t(hp.back()) + 1, make_int4(0, 0, 0, 0));
+    for (int u = 1; u < nuniq[s]; ++u)
+      for (int a = 0; a < nex[s][u]; ++a)
+        he[hpos[excs[s][off[s][u] + a]]++] =
+            make_int4(nex[s][u] | a << 8, off[s][u], io[u], u);
+    AFQMC_TRY(to_device(&h->hrow[s], hp.data(), hp.size()));
+    AFQMC_TRY(to_device(&h->hent[s], he.data(), he.size()));
     // table indexing of the excitations
     std::vector<int> hrow(nel[s], -1), vcol(nact[s], -1), hlv, vlv;
     for (int u = 1; u < nuniq[s]; ++u)
@@ -2071,10 +2251,28 @@ extern "C" int afqmc_phmsd_density_matrix(afqmc_phmsd h, const afqmc_c128* wbuf,
   cudaGetDevice(&prev);
   cudaSetDevice(h->device);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  // the density matrix needs only the per-walker Woodbury buffers (~0.5 MB per walker at
-  // nel = 30, nact = 70, 2000 excitations): blocks of up to 512 walkers
-  const int Wb = block > 0 ? (block < W ? block : W) : (W < 512 ? W : 512);
+  // the density matrix needs only the per-walker Woodbury buffers: blocks of at least 512 walkers,
+  // more as far as they fit 512 MiB (0.5 MB a walker at nel = 30, nact = 70, 2000 excitations;
+  // 20 KB at nel = 7, nact = 15, where 1536 walkers in one block take a third of the launches)
+  const size_t na = std::max(h->nact[0], h->nact[1]), ne = std::max(h->nel[0], h->nel[1]);
+  const size_t per_walker =
+      sizeof(c128) * (2 * ne * h->M + 4 * na * ne + ne * ne + h->nuniq[0] + h->nuniq[1] +
+                      2 * std::max(h->nuniq[0], h->nuniq[1]) +
+                      (3 * size_t(std::max(h->ninv[0], h->ninv[1])) + 1) / 2 + 2);
+  const size_t fit = std::min<size_t>(std::max<size_t>(512, (size_t(512) << 20) / per_walker),
+                                      65535);
+  int Wb = block > 0 ? (block < W ? block : W) : int(std::min<size_t>(W, fit));
+  // where more than 512 walkers' buffers cannot be had (a capture under way, memory taken): 512
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &cap);
+  if (block <= 0 && cap != cudaStreamCaptureStatusNone && h->capCore < Wb)
+    Wb = std::min(Wb, std::max(512, h->capCore));
   int st = phmsd_core_scratch(h, Wb);
+  if (st == AFQMC_ERR_ALLOC && block <= 0 && Wb > 512) {
+    cudaGetLastError();
+    Wb = 512;
+    st = phmsd_core_scratch(h, Wb);
+  }
   if (st) {
     cudaSetDevice(prev);
     return st;
@@ -2121,8 +2319,8 @@ extern "C" int afqmc_phmsd_density_matrix(afqmc_phmsd h, const afqmc_c128* wbuf,
                         N, na);
         AFQMC_CUDA_TRY(cudaFuncSetAttribute(phmsd_R_kernel,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(rsm)));
-        phmsd_R_kernel<<<nb, PHR_THREADS, rsm, s>>>(h->eQ[sp], h->refc[sp], h->uoff[sp],
-                                                    h->unex[sp], h->uexc[sp], h->uinv[sp], h->INV,
+        phmsd_R_kernel<<<nb, PHR_THREADS, rsm, s>>>(h->eQ[sp], h->refc[sp], h->hrow[sp],
+                                                    h->hent[sp], h->uexc[sp], h->INV,
                                                     h->ninv[sp], h->wgt, nu, nb, N, na, h->Rfull);
         AFQMC_TRY(launch_status("phmsd_R_kernel"));
         // G_s = R^T G_ref  (rows of this spin's active orbitals)
