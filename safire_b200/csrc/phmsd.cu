@@ -727,8 +727,8 @@ __global__ void __launch_bounds__(PH_THREADS) excited_1body_all_kernel(
 template <int NEX, int NG, typename C>
 __device__ __forceinline__ void excited_terms(const int* __restrict__ e4,
                                               const C* __restrict__ Qg, int es, const C* Sf,
-                                              const C* SU, int nv, int sfs, int sus, int ng,
-                                              const C* f0, C* exg, C* kng) {
+                                              const C* SU, int nv, int sfs, int sus,
+                                              const C (&f0)[NG], C (&exg)[NG], C (&kng)[NG]) {
   using R = decltype(f0[0].x);
   C Qi[NEX * NEX];  // the determinant's Woodbury inverse, in the working precision
 #pragma unroll
@@ -740,9 +740,9 @@ __device__ __forceinline__ void excited_terms(const int* __restrict__ e4,
     uo[a] = e4[(2 * NEX + a) * es] * nv;
     pc[a] = e4[(3 * NEX + a) * es];
   }
-#pragma unroll
-  for (int g = 0; g < NG; ++g) {
-    if (g >= ng) break;
+  constexpr int UNROLL_G = NEX > 4 ? 1 : NG;
+#pragma unroll UNROLL_G
+  for (int g = 0; g < NG; ++g) {  // past the group's indices: tables nobody wrote, unused sums
     const C* Sg = Sf + g * sfs;
     const C* Ug = SU + g * sus;
     C P[NEX][NEX];
@@ -753,13 +753,13 @@ __device__ __forceinline__ void excited_terms(const int* __restrict__ e4,
 #pragma unroll
       for (int q = 0; q < NEX; ++q) {
         sv[q] = Sg[so[a] + pc[q]];
-        d = cadd(d, cmul(Qi[a * NEX + q], Ug[uo[a] + pc[q]]));
+        d = cfma(Qi[a * NEX + q], Ug[uo[a] + pc[q]], d);
       }
 #pragma unroll
       for (int b = 0; b < NEX; ++b) {
         C acc = czero<C>();
 #pragma unroll
-        for (int q = 0; q < NEX; ++q) acc = cadd(acc, cmul(sv[q], Qi[b * NEX + q]));
+        for (int q = 0; q < NEX; ++q) acc = cfma(sv[q], Qi[b * NEX + q], acc);
         P[a][b] = acc;
       }
     }
@@ -767,21 +767,22 @@ __device__ __forceinline__ void excited_terms(const int* __restrict__ e4,
 #pragma unroll
     for (int a = 0; a < NEX; ++a) {
       tr = cadd(tr, P[a][a]);
-      pp = cadd(pp, cmul(P[a][a], P[a][a]));
+      pp = cfma(P[a][a], P[a][a], pp);
 #pragma unroll
-      for (int b = a + 1; b < NEX; ++b) off = cadd(off, cmul(P[a][b], P[b][a]));
+      for (int b = a + 1; b < NEX; ++b) off = cfma(P[a][b], P[b][a], off);
     }
     exg[g] = cadd(cadd(pp, cscale(off, R(2))), cscale(d, R(2)));
     kng[g] = cadd(f0[g], tr);
   }
 }
 
-// nex > 4 is rare: out of line, so that its larger frame stays out of the common path
+// nex > 4 is rare: out of line and in kernels of its own (RARE), so that its larger frame stays out
+// of the common path
 template <int NEX, int NG, typename C>
 __device__ __noinline__ void excited_terms_rare(const int* e4, const C* Qi, int es, const C* Sf,
-                                                const C* SU, int nv, int sfs, int sus, int ng,
-                                                const C* f0, C* exg, C* kng) {
-  excited_terms<NEX, NG, C>(e4, Qi, es, Sf, SU, nv, sfs, sus, ng, f0, exg, kng);
+                                                const C* SU, int nv, int sfs, int sus,
+                                                const C (&f0)[NG], C (&exg)[NG], C (&kng)[NG]) {
+  excited_terms<NEX, NG, C>(e4, Qi, es, Sf, SU, nv, sfs, sus, f0, exg, kng);
 }
 
 // One product of the tables: out[k][c] = sum_j a[r_k][sel_j] b[j][c] over the rows k < nrows
@@ -815,8 +816,8 @@ __device__ __forceinline__ void table_product(const C* a, int lda, const int* ro
 #pragma unroll
       for (int r = 0; r < RT; ++r) {
         const C x = ar[r][sj];
-        acc0[r] = cadd(acc0[r], cmul(x, b0));
-        acc1[r] = cadd(acc1[r], cmul(x, b1));
+        acc0[r] = cfma(x, b0, acc0[r]);
+        acc1[r] = cfma(x, b1, acc1[r]);
       }
     }
 #pragma unroll
@@ -871,7 +872,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // Woodbury inverses in the working type; uhdr[u] = {nex, base of u in uexc4, base of u in INVc,
 // stride es}: field entry k of excitation u at base + k es (es = 1: one excitation's entries
 // together; es = the shell's size: structure-of-arrays, consecutive excitations adjacent).
-template <typename R, int NG, typename TW>
+template <typename R, int NG, typename TW, bool RARE>
 __global__ void __launch_bounds__(PHX_THREADS, sizeof(R) == 4 ? 2 : 1) excited_energy_tables_kernel(
     const TW* __restrict__ Twina, const c128* __restrict__ QQ0, const int* __restrict__ refc,
     const int* __restrict__ hl, const int* __restrict__ vl, int nh, int nv,
@@ -925,7 +926,7 @@ __global__ void __launch_bounds__(PHX_THREADS, sizeof(R) == 4 ? 2 : 1) excited_e
   for (int g = 0; g < NG; ++g) {
     f0w[g] = czero<C>();
     f00[g] = cmk(0, 0);
-    if (g >= ng) break;
+    if (g >= ng) continue;
     const int n = n0 + g;
     C* Tn = (g & 1) ? Tb1 : Tb0;
     C* Sg = Sf + g * sfs;
@@ -977,28 +978,42 @@ __global__ void __launch_bounds__(PHX_THREADS, sizeof(R) == 4 ? 2 : 1) excited_e
     const int* e4 = uexc4 + hd.y;
     const C* Qi = Iw + hd.z;
     C exw[NG], knw[NG];
+    auto rare = [&]() {
+      C e5[NG], k5[NG];  // out-of-line results by address: apart, so that the common ones need none
+      switch (hd.x) {
+        case 5: excited_terms_rare<5, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, f0w, e5, k5); break;
+        case 6: excited_terms_rare<6, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, f0w, e5, k5); break;
+        case 7: excited_terms_rare<7, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, f0w, e5, k5); break;
+        default: excited_terms_rare<8, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, f0w, e5, k5); break;
+      }
+#pragma unroll
+      for (int g = 0; g < NG; ++g) {
+        exw[g] = e5[g];
+        knw[g] = k5[g];
+      }
+    };
     switch (hd.x) {
-      case 1: excited_terms<1, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, ng, f0w, exw, knw); break;
-      case 2: excited_terms<2, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, ng, f0w, exw, knw); break;
-      case 3: excited_terms<3, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, ng, f0w, exw, knw); break;
-      case 4: excited_terms<4, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, ng, f0w, exw, knw); break;
-      case 5: excited_terms_rare<5, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, ng, f0w, exw, knw); break;
-      case 6: excited_terms_rare<6, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, ng, f0w, exw, knw); break;
-      case 7: excited_terms_rare<7, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, ng, f0w, exw, knw); break;
-      default: excited_terms_rare<8, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, ng, f0w, exw, knw); break;
+      case 1: excited_terms<1, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, f0w, exw, knw); break;
+      case 2: excited_terms<2, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, f0w, exw, knw); break;
+      case 3: excited_terms<3, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, f0w, exw, knw); break;
+      case 4: excited_terms<4, NG, C>(e4, Qi, hd.w, Sf, SU, nv, sfs, sus, f0w, exw, knw); break;
+      default:
+        if constexpr (RARE) rare();
+        break;
     }
     c128 exu = cmk(0, 0), eju = cmk(0, 0);
     const size_t o = (size_t(u) * W + w) * nchol + n0;
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
-      if (g >= ng) break;
-      const c128 kn = to_cx<c128>(knw[g]);
-      exu = cadd(exu, to_cx<c128>(exw[g]));
-      eju = cadd(eju, csub(cmul(kn, kn), f00[g]));
-      if (cross)
-        ejc = cadd(ejc, cmul(to_cx<c128>(cross[o + g]), kn));
-      else
-        KE[o + g] = to_cx<TW>(kn);
+      if (g < ng) {
+        const c128 kn = to_cx<c128>(knw[g]);
+        exu = cadd(exu, to_cx<c128>(exw[g]));
+        eju = cadd(eju, csub(cmul(kn, kn), f00[g]));
+        if (cross)
+          ejc = cadd(ejc, cmul(to_cx<c128>(cross[o + g]), kn));
+        else
+          KE[o + g] = to_cx<TW>(kn);
+      }
     }
     exs = cadd(exs, cmul(wu, exu));
     ejs = cadd(ejs, cmul(wu, eju));
@@ -1060,7 +1075,7 @@ __global__ void couple_ke_kernel(const int* __restrict__ seg, const int* __restr
   for (int n = threadIdx.x; n < nchol; n += blockDim.x) {
     c128 acc = cmk(0, 0);
     for (int j = 0; j < j1 - j0; ++j)
-      acc = cadd(acc, cmul(f[j], to_cx<c128>(KEr[(size_t(uu[j]) * W + w) * nchol + n])));
+      acc = cfma(f[j], to_cx<c128>(KEr[(size_t(uu[j]) * W + w) * nchol + n]), acc);
     KT* o = KEd + (size_t(d) * W + w) * nchol + n;
     if (single)
       *o = to_cx<KT>(acc);
@@ -2120,15 +2135,24 @@ int phmsd_reference_and_excited(afqmc_phmsd h, cudaStream_t s, int sp, int nb, d
     };
     const c64* inv32 = reinterpret_cast<const c64*>(h->INV32);
     const c64* tw64 = reinterpret_cast<const c64*>(h->Twina);
+    const bool rare = !h->sh_nex[sp].empty() &&
+                      *std::max_element(h->sh_nex[sp].begin(), h->sh_nex[sp].end()) > 4;
+    auto go_ng = [&](auto r, const auto* tw, const auto* inv) -> int {
+      using R = decltype(r);
+      using TW = std::remove_const_t<std::remove_pointer_t<decltype(tw)>>;
+      if (ngr == 4)
+        return rare ? go(excited_energy_tables_kernel<R, 4, TW, true>, tw, inv)
+                    : go(excited_energy_tables_kernel<R, 4, TW, false>, tw, inv);
+      return rare ? go(excited_energy_tables_kernel<R, 1, TW, true>, tw, inv)
+                  : go(excited_energy_tables_kernel<R, 1, TW, false>, tw, inv);
+    };
+    const c128* twd = h->Twina;
     if (mixed && h->twina64[sp])
-      AFQMC_TRY(ngr == 4 ? go(excited_energy_tables_kernel<float, 4, c64>, tw64, inv32)
-                         : go(excited_energy_tables_kernel<float, 1, c64>, tw64, inv32));
+      AFQMC_TRY(go_ng(0.f, tw64, inv32));
     else if (mixed)
-      AFQMC_TRY(ngr == 4 ? go(excited_energy_tables_kernel<float, 4, c128>, h->Twina, inv32)
-                         : go(excited_energy_tables_kernel<float, 1, c128>, h->Twina, inv32));
+      AFQMC_TRY(go_ng(0.f, twd, inv32));
     else
-      AFQMC_TRY(ngr == 4 ? go(excited_energy_tables_kernel<double, 4, c128>, h->Twina, h->INV)
-                         : go(excited_energy_tables_kernel<double, 1, c128>, h->Twina, h->INV));
+      AFQMC_TRY(go_ng(0.0, twd, static_cast<const c128*>(h->INV)));
     AFQMC_TRY(launch_status("excited_energy_tables_kernel"));
     reference_from_tables_kernel<<<(nb + 127) / 128, 128, 0, s>>>(h->Swia, h->refc[sp], N, na, E0,
                                                                   h->eOv, REF, nb, E);
