@@ -42,7 +42,7 @@ enum Epi : int {
 
 // Symmetric vHS tiles: the BN = 128 columns of a tile are the (i, k) pairs of an 8 x 16 block,
 // column j = 8-row offset * 16 + 16-column offset; only blocks holding some i <= k are computed.
-constexpr int SYM_IB = 8, SYM_KB = 16, SYM_MAXIB = 32;
+constexpr int SYM_IB = 8, SYM_KB = 16, SYM_MAXKB = 16;
 
 struct TcParams {
   CUtensorMap a[4];
@@ -66,19 +66,22 @@ struct TcParams {
   // EPI_VHS / EPI_VHS_SYM with out_f16: the output planes are FP16 holding value * out_sc[row]
   int out_f16;
   const float* out_sc;
-  // EPI_VHS_SYM: sym_pre[a] = tiles of the i blocks before block a (a = 0..sym_nib), sym_nkb =
-  // number of k blocks; block a covers the top sym_pre[a+1] - sym_pre[a] k blocks
-  int sym_nib, sym_nkb;
-  int sym_pre[SYM_MAXIB + 1];
+  // EPI_VHS_SYM: sym_pre[c] = tiles of the k blocks before block c (c = 0..sym_nkb); block c meets
+  // the i blocks 0 .. sym_pre[c+1] - sym_pre[c] - 1
+  int sym_nkb;
+  int sym_pre[SYM_MAXKB + 1];
   unsigned* err;
 };
 
-// tile nt of the symmetric vHS -> (i block a, k block c)
+// tile nt of the symmetric vHS -> (i block a, k block c), the i block fastest: the two 16-byte halves
+// of a mirrored row's 32-byte sector come from neighbouring tiles, which run at the same time and
+// meet in the L2 cache.  1024 walkers, M = 200, 1600 vectors (FP16 planes): 777 us with 16-byte stores
+// on 16-byte rows and the k block fastest, 611 us with this order and whole sectors; 354 us with the
+// stores left out, so the stores are still what bounds it.
 __device__ __forceinline__ void sym_tile(const TcParams& p, int nt, int& a, int& c) {
-  a = 0;
-  while (a + 1 < p.sym_nib && p.sym_pre[a + 1] <= nt) ++a;
-  const int cnt = p.sym_pre[a + 1] - p.sym_pre[a];
-  c = p.sym_nkb - cnt + (nt - p.sym_pre[a]);
+  c = 0;
+  while (c + 1 < p.sym_nkb && p.sym_pre[c + 1] <= nt) ++c;
+  a = nt - p.sym_pre[c];
 }
 
 template <bool A_CPLX, bool B_CPLX, int BN, int STAGES>
@@ -123,21 +126,31 @@ __device__ __forceinline__ void tc_tile(long t, int MT, int NT, int order, int& 
 // each value goes to V[w][i][k] (i <= k) and V[w][k][i] (i < k), the real then the imaginary
 // part, so that a thread holds a whole 8 x 16 block (128 registers) and writes rows of 16 (direct)
 // and 8 (mirrored) consecutive floats.
+// 32 bytes to a 32-byte boundary: a whole sector
+__device__ __forceinline__ void store_sector(void* dst, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(v[0]), "r"(v[1]),
+               "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
+// v[0..NRUN): consecutive values of one row at idx (a multiple of NRUN past a 32-byte boundary); only
+// offsets [first, last) are written (fully unrolled: v stays in registers)
 template <int NRUN>
 __device__ __forceinline__ void store_run(float* hi, float* lo, long idx, const float* v,
                                           int first, int last, float alpha) {
-  // v[0..NRUN): consecutive values of one row at idx; only offsets [first, last) are written
-  // (fully unrolled: v stays in registers)
   if (first == 0 && last == NRUN) {
 #pragma unroll
-    for (int j = 0; j < NRUN; j += 4) {
-      float4 h, l;
-      tc::tf32_split(alpha * v[j + 0], h.x, l.x);
-      tc::tf32_split(alpha * v[j + 1], h.y, l.y);
-      tc::tf32_split(alpha * v[j + 2], h.z, l.z);
-      tc::tf32_split(alpha * v[j + 3], h.w, l.w);
-      *reinterpret_cast<float4*>(hi + idx + j) = h;
-      *reinterpret_cast<float4*>(lo + idx + j) = l;
+    for (int j = 0; j < NRUN; j += 8) {
+      uint32_t h[8], l[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        float a, b;
+        tc::tf32_split(alpha * v[j + t], a, b);
+        h[t] = __float_as_uint(a);
+        l[t] = __float_as_uint(b);
+      }
+      store_sector(hi + idx + j, h);
+      store_sector(lo + idx + j, l);
     }
   } else {
 #pragma unroll
@@ -151,13 +164,22 @@ template <int NRUN>
 __device__ __forceinline__ void store_run16(__half* hi, __half* lo, long idx, const float* v,
                                             int first, int last, float alpha) {
   if (first == 0 && last == NRUN) {
+    uint32_t h[NRUN / 2], l[NRUN / 2];
 #pragma unroll
-    for (int j = 0; j < NRUN; j += 8) {
-      __align__(16) __half h[8], l[8];
-#pragma unroll
-      for (int t = 0; t < 8; ++t) tc::f16_split(alpha * v[j + t], h[t], l[t]);
-      *reinterpret_cast<uint4*>(hi + idx + j) = *reinterpret_cast<const uint4*>(h);
-      *reinterpret_cast<uint4*>(lo + idx + j) = *reinterpret_cast<const uint4*>(l);
+    for (int j = 0; j < NRUN; j += 2) {
+      __half2 a, b;
+      tc::f16_split(alpha * v[j], a.x, b.x);
+      tc::f16_split(alpha * v[j + 1], a.y, b.y);
+      h[j / 2] = *reinterpret_cast<const uint32_t*>(&a);
+      l[j / 2] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    if constexpr (NRUN == 16) {
+      store_sector(hi + idx, h);
+      store_sector(lo + idx, l);
+    } else {
+      static_assert(NRUN == 8, "a sector or half of one");
+      *reinterpret_cast<uint4*>(hi + idx) = make_uint4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<uint4*>(lo + idx) = make_uint4(l[0], l[1], l[2], l[3]);
     }
   } else {
 #pragma unroll
@@ -201,7 +223,8 @@ __device__ __forceinline__ void vhs_sym_epilogue(const TcParams& p, uint32_t tro
       const int i = i0 + a;
       if (i >= M) break;
       const int first = i > k0 ? i - k0 : 0;
-      const int last = M - k0 < SYM_KB ? M - k0 : SYM_KB;
+      // a row's padding takes the zeros past M
+      const int last = p.out_ld - k0 < SYM_KB ? M - k0 : SYM_KB;
       if (first >= last) continue;
       if (p.out_f16)
         store_run16<SYM_KB>(hi16, lo16, wb + long(i) * p.out_ld + k0, v[a], first, last, alpha);
@@ -566,13 +589,15 @@ struct Planes {
   }
 };
 
-int alloc_planes(Planes& P, int nplanes, long batch, long rows, long k, int esize = 4) {
+// Rows start on row_bytes: 16 (TMA strides), or 32 where whole sectors of a row are stored at a time.
+int alloc_planes(Planes& P, int nplanes, long batch, long rows, long k, int esize = 4,
+                 int row_bytes = 16) {
   P.nplanes = nplanes;
   P.esize = esize;
   P.batch = batch;
   P.rows = rows;
   P.k = k;
-  const long align = 16 / esize;  // rows start on 16 bytes (TMA strides)
+  const long align = row_bytes / esize;
   P.ld = (k + align - 1) / align * align;
   for (int q = 0; q < nplanes; ++q) {
     cudaError_t e = cudaMalloc(&P.p[q], size_t(esize) * P.elems());
@@ -1022,7 +1047,7 @@ int mixed_ham_create(MixedHam** out, const EnergyArgs& a, cudaStream_t s) {
   }
   // real orbitals make every Cholesky vector symmetric (L_n[i][k] = L_n[k][i]); then V_w is
   // complex symmetric and vHS computes only the i <= k half
-  if (a.nspin_H2 == 1 && a.M <= SYM_IB * SYM_MAXIB)
+  if (a.nspin_H2 == 1 && a.M <= SYM_KB * SYM_MAXKB)
     AFQMC_TRY(likn_is_symmetric(a.Likn, a.M, a.Nc, &m->likn_sym));
   // FP16 split: 16-byte rows of FP16 planes (M, Nc multiples of 8), one spin block of L, a real
   // trial and at most 50 electrons per spin (the fused exchange)
@@ -1237,31 +1262,35 @@ int vbias_mixed(cudaStream_t s, MixedHam* m, const c128* G, long ldG, c128* v, i
 // propagation reads them as its A operand.  When V is a complex128 output (the C-ABI call
 // afqmc_ham_vhs) the planes are re-assembled into V afterwards.
 namespace {
+// V planes [w][i][k] (row pitch ld) -> complex128 [W][M*M]; n = W M M
 __global__ void planes_to_c128_kernel(const float* __restrict__ rh, const float* __restrict__ rl,
                                       const float* __restrict__ ih, const float* __restrict__ il,
-                                      long n, c128* __restrict__ out) {
+                                      long n, int M, long ld, c128* __restrict__ out) {
   long e = blockIdx.x * long(blockDim.x) + threadIdx.x;
-  if (e < n) out[e] = cmk(double(rh[e]) + double(rl[e]), double(ih[e]) + double(il[e]));
+  if (e >= n) return;
+  const long r = e / M, d = r * ld + (e - r * M);
+  out[e] = cmk(double(rh[d]) + double(rl[d]), double(ih[d]) + double(il[d]));
 }
 
-// FP16 V planes -> complex128 [W][M*M]: (hi + lo) * v_inv[w]
+// the same from FP16 planes: (hi + lo) * v_inv[w]
 __global__ void planes16_to_c128_kernel(const __half* __restrict__ rh,
                                         const __half* __restrict__ rl,
                                         const __half* __restrict__ ih,
-                                        const __half* __restrict__ il, long n, long per_walker,
+                                        const __half* __restrict__ il, long n, int M, long ld,
                                         const float* __restrict__ v_inv, c128* __restrict__ out) {
   long e = blockIdx.x * long(blockDim.x) + threadIdx.x;
   if (e >= n) return;
-  const double f = v_inv[e / per_walker];
-  out[e] = cmk((double(__half2float(rh[e])) + double(__half2float(rl[e]))) * f,
-               (double(__half2float(ih[e])) + double(__half2float(il[e]))) * f);
+  const long r = e / M, d = r * ld + (e - r * M);
+  const double f = v_inv[r / M];
+  out[e] = cmk((double(__half2float(rh[d])) + double(__half2float(rl[d]))) * f,
+               (double(__half2float(ih[d])) + double(__half2float(il[d]))) * f);
 }
 
 int ensure_v_buffers(MixedHam* m, int W) {
   if (m->V.batch >= W) return AFQMC_OK;
   AFQMC_CUDA_TRY(cudaDeviceSynchronize());
   free_planes(m->V);
-  return alloc_planes(m->V, 4, W, m->M, m->M);
+  return alloc_planes(m->V, 4, W, m->M, m->M, 4, 32);
 }
 
 int ensure_v_buffers16(MixedHam* m, int W) {
@@ -1271,7 +1300,7 @@ int ensure_v_buffers16(MixedHam* m, int W) {
   if (m->v_inv) cudaFree(m->v_inv);
   if (m->v_sc) cudaFree(m->v_sc);
   m->v_inv = m->v_sc = nullptr;
-  AFQMC_TRY(alloc_planes(m->V16, 4, W, m->M, m->M, 2));
+  AFQMC_TRY(alloc_planes(m->V16, 4, W, m->M, m->M, 2, 32));
   AFQMC_CUDA_TRY(cudaMalloc(&m->v_inv, sizeof(float) * W));
   AFQMC_CUDA_TRY(cudaMalloc(&m->v_sc, sizeof(float) * W));
   return AFQMC_OK;
@@ -1353,16 +1382,14 @@ int vhs_planes(cudaStream_t s, MixedHam* m, const c128* X, int W, double a) {
     for (int q = 0; q < 2; ++q)
       AFQMC_TRY(make_plane_map_3d_es(&p.b[q], Lp.p[q], Lp.esize, m->Nc, M, Lp.ld, M,
                                      long(M) * Lp.ld, SYM_KB, SYM_IB));
-    p.sym_nib = ceil_div(M, SYM_IB);
     p.sym_nkb = ceil_div(M, SYM_KB);
+    const int nib = ceil_div(M, SYM_IB);
     p.sym_pre[0] = 0;
-    for (int ab = 0; ab < p.sym_nib; ++ab) {
-      int cnt = 0;
-      for (int cb = 0; cb < p.sym_nkb; ++cb)
-        if (cb * SYM_KB + SYM_KB - 1 >= ab * SYM_IB) ++cnt;
-      p.sym_pre[ab + 1] = p.sym_pre[ab] + cnt;
+    for (int cb = 0; cb < p.sym_nkb; ++cb) {  // i blocks that hold some i <= k
+      const int cnt = (cb * SYM_KB + SYM_KB - 1) / SYM_IB + 1;
+      p.sym_pre[cb + 1] = p.sym_pre[cb] + (cnt < nib ? cnt : nib);
     }
-    p.m = W; p.n = p.sym_pre[p.sym_nib] * 128; p.k = m->Nc;
+    p.m = W; p.n = p.sym_pre[p.sym_nkb] * 128; p.k = m->Nc;
     p.alpha = cmk(a, 0);
     const Planes& Vo = v16 ? m->V16 : m->V;
     for (int q = 0; q < 4; ++q) p.out[q] = Vo.p[q];
@@ -1399,27 +1426,17 @@ int vhs_mixed(cudaStream_t s, MixedHam* m, const c128* X, c128* V, int W, double
     return AFQMC_ERR_UNSUPPORTED;
   }
   AFQMC_TRY(vhs_planes(s, m, X, W, a));
-  if (V && m->v_is_f16) {
-    const long n = long(W) * m->M * m->M;
-    if (m->V16.ld != m->M) {
-      set_error_detail("vhs_mixed: padded V planes cannot be copied out");
-      return AFQMC_ERR_UNSUPPORTED;
-    }
-    planes16_to_c128_kernel<<<ceil_div(n, 256), 256, 0, s>>>(
-        m->V16.h(0), m->V16.h(1), m->V16.h(2), m->V16.h(3), n, long(m->M) * m->M, m->v_inv, V);
+  if (!V) return AFQMC_OK;
+  const long n = long(W) * m->M * m->M;
+  if (m->v_is_f16) {
+    planes16_to_c128_kernel<<<ceil_div(n, 256), 256, 0, s>>>(m->V16.h(0), m->V16.h(1), m->V16.h(2),
+                                                             m->V16.h(3), n, m->M, m->V16.ld,
+                                                             m->v_inv, V);
     return launch_status("planes16_to_c128_kernel");
   }
-  if (V) {
-    const long n = long(W) * m->M * m->M;
-    if (m->V.ld != m->M) {
-      set_error_detail("vhs_mixed: padded V planes cannot be copied out");
-      return AFQMC_ERR_UNSUPPORTED;
-    }
-    planes_to_c128_kernel<<<ceil_div(n, 256), 256, 0, s>>>(m->V.p[0], m->V.p[1], m->V.p[2],
-                                                           m->V.p[3], n, V);
-    AFQMC_TRY(launch_status("planes_to_c128_kernel"));
-  }
-  return AFQMC_OK;
+  planes_to_c128_kernel<<<ceil_div(n, 256), 256, 0, s>>>(m->V.p[0], m->V.p[1], m->V.p[2], m->V.p[3],
+                                                         n, m->M, m->V.ld, V);
+  return launch_status("planes_to_c128_kernel");
 }
 
 int taylor_fused_tc(cudaStream_t s, int esize, const void* const P1p[2], const void* const Vp[4],
