@@ -116,3 +116,26 @@ def test_vhs_vbias_shapes(cuda, W, M, Nc):
     want = 0.2 * (G.real @ Lnak.T + 1j * (G.imag @ Lnak.T))
     scale = 0.2 * np.max(np.abs(G)) * np.max(np.abs(Lnak))
     assert np.max(np.abs(to_host(v) - want)) < 20 * N * M * EPS * scale
+
+
+@pytest.mark.parametrize("N", [1, 5, 8, 10, 16, 17, 20, 25, 30, 32, 33, 40, 41, 50])
+@pytest.mark.parametrize("fmt", [1, 2])  # TF32, FP16 split
+def test_exchange_tiles(cuda, N, fmt):
+    """The tensor-core exchange at every tile layout, ragged in walkers and vectors, against the
+    complex128 energy.  Operands keep 22 bits and the sums run in FP32: 2^-21 per element of the
+    rows' magnitude, a few 1e-6 relative of sums that hardly cancel (their diagonal leads)."""
+    from safire_b200 import afqmc as A
+    M, Nc, W = 104, 56, 29
+    rs = np.random.default_rng(N)
+    L = 0.1 * rs.standard_normal((M, M, Nc))
+    ham = _ham(M, N, Nc, L + L.transpose(1, 0, 2))
+    ham.set_split_format(fmt)
+    G = to_dev(rand_c(rs, W, N * M, scale=0.05)
+               + np.eye(N, M).reshape(-1)[None] * (1 + 0.1 * rs.random((W, 1))))
+    E, R = (torch.zeros((W, 3), dtype=torch.complex128, device=cuda) for _ in range(2))
+    ham.energy(E, G, precision=A.PREC_MIXED)
+    ham.energy(R, G)
+    assert ham.device_error_flag() == 0
+    E, R = to_host(E), to_host(R)
+    for c in (1, 2):
+        assert np.max(np.abs(E[:, c] - R[:, c])) < 2e-5 * np.max(np.abs(R[:, c])), c
