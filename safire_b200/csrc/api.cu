@@ -98,7 +98,9 @@ struct afqmc_ham_s {
   double* Lnak_r[2] = {nullptr, nullptr};
   c128* haj = nullptr;                  // [nel_tot][M]
   c128* PsiT = nullptr;                 // [nel_tot][M]
+  double* PsiT_r = nullptr;             // the same as real numbers, if trial_real
   c128* PsiH = nullptr;                 // [M][nel_s] per spin, concatenated (initial walker)
+  const double* psi_r(int sp) const { return PsiT_r ? PsiT_r + long(el_off[sp]) * M : nullptr; }
   std::vector<c128> hij_h;              // [nspin_H1][M][M]
   std::vector<double> vexx_h;           // [nspin_H2][M][M]
   MixedHam* mixed = nullptr;            // tensor-core copies (built on first mixed call)
@@ -112,7 +114,7 @@ struct afqmc_ham_s {
       dfree(Lnak_r[s]);
     }
     dfree(haj);
-    dfree(PsiT);
+    dfree(PsiT); dfree(PsiT_r);
     dfree(PsiH);
     if (mixed) mixed_ham_destroy(mixed);
   }
@@ -186,10 +188,15 @@ struct afqmc_nomsd_s {
   int device = 0;
   std::vector<afqmc_ham_s*> hams;
   std::vector<c128> ci;
+  double* PsiTall_r = nullptr;  // the same as real numbers, if every determinant's trial is real
   c128 *PsiTall = nullptr, *dcc = nullptr, *dlc = nullptr;  // conj(ci), log conj(ci)
   c128 *Gc = nullptr, *ov = nullptr, *T = nullptr, *Ed = nullptr;  // energy (per determinant)
   c128 *Tb = nullptr, *Ttb = nullptr, *Gcb = nullptr, *ovd = nullptr, *wdd = nullptr;
   int capW = 0, wchunk = 0;
+  // element `off` of the stacked trials, real where they are real
+  const void* psi(long off) const {
+    return PsiTall_r ? static_cast<const void*>(PsiTall_r + off) : PsiTall + off;
+  }
   void free_bufs() {
     dfree(Gc); dfree(ov); dfree(T); dfree(Ed);
     dfree(Tb); dfree(Ttb); dfree(Gcb); dfree(ovd); dfree(wdd);
@@ -199,7 +206,7 @@ struct afqmc_nomsd_s {
   ~afqmc_nomsd_s() {
     DeviceGuard g(device);
     free_bufs();
-    dfree(PsiTall); dfree(dcc); dfree(dlc);
+    dfree(PsiTall); dfree(PsiTall_r); dfree(dcc); dfree(dlc);
   }
 };
 
@@ -562,6 +569,13 @@ int ham_trial_setup(afqmc_ham_s* h, const afqmc_c128* hij, int nspin_H1, const c
   AFQMC_TRY(dalloc(&h->PsiT, size_t(h->nel_tot) * M));
   if (h->nel_tot)
     AFQMC_CUDA_TRY(cudaMemcpy(h->PsiT, psi, sizeof(c128) * h->nel_tot * M, cudaMemcpyHostToDevice));
+  if (real && h->nel_tot) {
+    std::vector<double> pr(size_t(h->nel_tot) * M);
+    for (size_t e = 0; e < pr.size(); ++e) pr[e] = psi[e].x;
+    AFQMC_TRY(dalloc(&h->PsiT_r, pr.size()));
+    AFQMC_CUDA_TRY(cudaMemcpy(h->PsiT_r, pr.data(), sizeof(double) * pr.size(),
+                              cudaMemcpyHostToDevice));
+  }
   // PsiH: per spin [M][nel_s] = conj(PsiT_s)^T, concatenated spin blocks
   {
     std::vector<c128> ph(size_t(h->nel_tot) * M);
@@ -1086,7 +1100,7 @@ int wfn_density_matrix(afqmc_ham_s* h, afqmc_wset_s* ws, cudaStream_t s, c128* G
     const c128 scale = (h->walker_type == AFQMC_CLOSED) ? cmk(2, 0) : cmk(1, 0);
     AFQMC_TRY(mixed_density_matrix(s, h->PsiT + long(h->el_off[sp]) * h->M, ws->buf + ws->offS(sp),
                                    ws->walker_size, G + long(h->el_off[sp]) * h->M, ldG, ovlp, W,
-                                   h->M, Ns, true, workT, nullptr, scale, cmk(0, 0)));
+                                   h->M, Ns, true, workT, nullptr, scale, cmk(0, 0), h->psi_r(sp)));
   }
   return AFQMC_OK;
 }
@@ -1099,7 +1113,8 @@ int wfn_log_overlap(afqmc_ham_s* h, afqmc_wset_s* ws, cudaStream_t s, c128* ovlp
     if (Ns == 0) continue;
     const c128 scale = (h->walker_type == AFQMC_CLOSED) ? cmk(2, 0) : cmk(1, 0);
     AFQMC_TRY(log_overlap(s, h->PsiT + long(h->el_off[sp]) * h->M, ws->buf + ws->offS(sp),
-                          ws->walker_size, ovlp, W, h->M, Ns, workT, scale, cmk(0, 0)));
+                          ws->walker_size, ovlp, W, h->M, Ns, workT, scale, cmk(0, 0),
+                          h->psi_r(sp)));
   }
   return AFQMC_OK;
 }
@@ -1285,11 +1300,11 @@ int nomsd_overlaps(afqmc_nomsd md, afqmc_wset_s* ws, cudaStream_t s, int w0, int
     toff += long(md->wchunk) * nd * nsq;
     GemmParams p{};
     p.m = nd * Ns; p.n = Ns; p.k = int(M);
-    p.A = md->PsiTall + long(nd) * h0->el_off[sp] * M; p.lda = M; p.strideA = 0;
+    p.A = md->psi(long(nd) * h0->el_off[sp] * M); p.lda = M; p.strideA = 0;
     p.B = S0 + ws->offS(sp); p.ldb = Ns; p.strideB = ws->walker_size;
     p.C = Tsp; p.ldc = Ns; p.strideC = long(nd) * nsq;
     p.alpha = cmk(1, 0); p.beta = cmk(0, 0);
-    AFQMC_TRY(zgemm(s, wc, GN, false, GN, false, p));
+    AFQMC_TRY(zgemm(s, wc, GN, md->PsiTall_r != nullptr, GN, false, p));
     AFQMC_TRY(batched_logdet_inverse(s, Tsp, nsq, invert ? Tsp : nullptr, nsq, md->ovd, int(nb),
                                      Ns, invert, scale, cmk(0, 0)));
   }
@@ -1353,11 +1368,11 @@ int nomsd_density_matrix(afqmc_nomsd md, afqmc_wset_s* ws, cudaStream_t s, c128*
       // G[w][s] = PsiTall_s^T Gc[w]  (K = nd * N_s: the sum over determinants)
       GemmParams q{};
       q.m = int(M); q.n = int(M); q.k = nd * Ns;
-      q.A = md->PsiTall + long(nd) * h0->el_off[sp] * M; q.lda = M; q.strideA = 0;
+      q.A = md->psi(long(nd) * h0->el_off[sp] * M); q.lda = M; q.strideA = 0;
       q.B = Gcsp; q.ldb = M; q.strideB = long(nd) * Ns * M;
       q.C = Gw + sp * MM; q.ldc = M; q.strideC = per;
       q.alpha = cmk(1, 0); q.beta = cmk(0, 0);
-      AFQMC_TRY(zgemm(s, wc, GT, false, GN, false, q));
+      AFQMC_TRY(zgemm(s, wc, GT, md->PsiTall_r != nullptr, GN, false, q));
     }
   }
   return AFQMC_OK;
@@ -1410,11 +1425,18 @@ extern "C" int afqmc_nomsd_create(int ndet, const afqmc_ham* hams, const afqmc_c
   // 1e-12 in modulus enters the log overlap as 1e-12, NOMSD.cpp:303-316)
   const long M = h0->M;
   AFQMC_TRY(dalloc(&md->PsiTall, size_t(ndet) * (h0->nel_tot > 0 ? h0->nel_tot : 1) * M));
+  bool real = h0->nel_tot > 0;
+  for (int d = 0; d < ndet; ++d) real = real && hams[d]->PsiT_r;
+  if (real) AFQMC_TRY(dalloc(&md->PsiTall_r, size_t(ndet) * h0->nel_tot * M));
   for (int sp = 0; sp < h0->nspin; ++sp) {
     const long rows = long(h0->nel[sp]) * M;
     for (int d = 0; d < ndet && rows > 0; ++d)
       AFQMC_CUDA_TRY(cudaMemcpy(md->PsiTall + long(ndet) * h0->el_off[sp] * M + d * rows,
                                 hams[d]->PsiT + long(h0->el_off[sp]) * M, sizeof(c128) * rows,
+                                cudaMemcpyDeviceToDevice));
+    for (int d = 0; d < ndet && rows > 0 && real; ++d)
+      AFQMC_CUDA_TRY(cudaMemcpy(md->PsiTall_r + long(ndet) * h0->el_off[sp] * M + d * rows,
+                                hams[d]->PsiT_r + long(h0->el_off[sp]) * M, sizeof(double) * rows,
                                 cudaMemcpyDeviceToDevice));
   }
   std::vector<c128> cc(ndet), lc(ndet);

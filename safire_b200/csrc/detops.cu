@@ -801,30 +801,32 @@ int batched_logdet_inverse(cudaStream_t s, const c128* A, long strideA, c128* Ai
 // Mixed density matrix / log overlap
 // ---------------------------------------------------------------------------------------------
 int overlap_matrices(cudaStream_t s, const c128* PsiT, const c128* S, long ldS, c128* T, int W,
-                     int M, int N) {
+                     int M, int N, const double* PsiT_r) {
   // T_w = PsiT (N x M) * S_w (M x N)   (math::product(A,B,TNN), density_matrix.hpp:142)
   GemmParams p{};
   p.m = N; p.n = N; p.k = M;
-  p.A = PsiT; p.lda = M; p.strideA = 0;
+  p.A = PsiT_r ? (const void*)PsiT_r : (const void*)PsiT; p.lda = M; p.strideA = 0;
   p.B = S; p.ldb = N; p.strideB = ldS;
   p.C = T; p.ldc = N; p.strideC = long(N) * N;
   p.alpha = cmk(1, 0); p.beta = cmk(0, 0);
-  return zgemm(s, W, GN, false, GN, false, p);
+  return zgemm(s, W, GN, PsiT_r != nullptr, GN, false, p);
 }
 
 int log_overlap(cudaStream_t s, const c128* PsiT, const c128* S, long ldS, c128* ovlp, int W,
-                int M, int N, c128* work_T, c128 post_scale, c128 post_add) {
+                int M, int N, c128* work_T, c128 post_scale, c128 post_add,
+                const double* PsiT_r) {
   if (N == 0) return AFQMC_OK;
-  AFQMC_TRY(overlap_matrices(s, PsiT, S, ldS, work_T, W, M, N));
+  AFQMC_TRY(overlap_matrices(s, PsiT, S, ldS, work_T, W, M, N, PsiT_r));
   return batched_logdet_inverse(s, work_T, long(N) * N, nullptr, 0, ovlp, W, N, false, post_scale,
                                 post_add);
 }
 
 int mixed_density_matrix(cudaStream_t s, const c128* PsiT, const c128* S, long ldS, c128* G,
                          long ldG, c128* ovlp, int W, int M, int N, bool compact, c128* work_T,
-                         c128* work_NM, c128 post_scale, c128 post_add) {
+                         c128* work_NM, c128 post_scale, c128 post_add,
+                         const double* PsiT_r) {
   if (N == 0) return AFQMC_OK;
-  AFQMC_TRY(overlap_matrices(s, PsiT, S, ldS, work_T, W, M, N));
+  AFQMC_TRY(overlap_matrices(s, PsiT, S, ldS, work_T, W, M, N, PsiT_r));
   AFQMC_TRY(batched_logdet_inverse(s, work_T, long(N) * N, work_T, long(N) * N, ovlp, W, N, true,
                                    post_scale, post_add));
   // C = TNN^T * S^T  (product<'T','T'>, density_matrix.hpp:576): [N x M]

@@ -17,6 +17,7 @@ int launch_hn(cudaStream_t, int, const GemmParams&, const Shape&);
 int launch_rrt(cudaStream_t, int, const GemmParams&, const Shape&);
 int launch_nc(cudaStream_t, int, const GemmParams&, const Shape&);
 int launch_nh(cudaStream_t, int, const GemmParams&, const Shape&);
+int launch_rtn(cudaStream_t, int, const GemmParams&, const Shape&);
 int launch_nrt_sym(cudaStream_t, const GemmParams&, const Shape&);
 
 namespace {
@@ -109,6 +110,7 @@ int zgemm(cudaStream_t s, int batch, GemmTrans ta, bool a_real, GemmTrans tb, bo
   AFQMC_GEMM_CASE(false, false, false, true, false, true, launch_nrt)   // A * real B^T
   AFQMC_GEMM_CASE(true, false, false, true, false, false, launch_tt)    // A^T * B^T
   AFQMC_GEMM_CASE(true, false, false, false, false, false, launch_tn)   // A^T * B
+  AFQMC_GEMM_CASE(true, false, true, false, false, false, launch_rtn)   // real A^T * B
   AFQMC_GEMM_CASE(true, true, false, false, false, false, launch_hn)    // A^H * B
   AFQMC_GEMM_CASE(false, false, true, true, false, true, launch_rrt)    // real A * real B^T
   AFQMC_GEMM_CASE(false, false, false, false, true, false, launch_nc)   // A * conj(B)

@@ -118,6 +118,37 @@ def test_vhs_vbias_shapes(cuda, W, M, Nc):
     assert np.max(np.abs(to_host(v) - want)) < 20 * N * M * EPS * scale
 
 
+@pytest.mark.parametrize("M,N,W,ndet", [(9, 1, 3, 1), (17, 5, 40, 3), (64, 16, 9, 1), (75, 33, 30, 2),
+                                       (41, 20, 300, 2)])
+def test_real_trial(cuda, M, N, W, ndet):
+    """Overlaps and density matrices of a real trial take the products with a real matrix; one
+    element with the imaginary part 1e-300, which no sum can feel, takes the complex ones: the
+    results are the same bit for bit."""
+    from safire_b200 import afqmc as A
+    rs = np.random.default_rng(M)
+    L = np.zeros((M, M, 2))
+    hij = np.eye(M)[None].astype(complex)
+    S = to_dev(np.eye(M, N) + rand_c(rs, W, M, N, scale=0.3 / np.sqrt(M)))
+    out = []
+    psi = [np.linalg.qr(np.eye(M, N) + 0.3 * rs.standard_normal((M, N)) / np.sqrt(M))[0].T.astype(complex)
+           for _ in range(ndet)]
+    for im in (0.0, 1e-300):
+        hams = []
+        for P in psi:
+            P = P.copy()
+            P[0, 0] += 1j * im
+            hams.append(A.HamiltonianOperations(A.CLOSED, M, N, N, L[None], hij, 0.0, [P]))
+        wset = A.WalkerSet(A.CLOSED, M, N, N, W)
+        wset.init_from_trial(hams[0])
+        wset.SlaterMatrices(0).copy_(S)
+        t = A.NOMSDMulti(hams, np.arange(1.0, ndet + 1).astype(complex)) if ndet > 1 else A.NOMSD(hams[0])
+        lo = t.Log_Overlap(wset)
+        G, ov = t.MixedDensityMatrix(wset)
+        out.append([to_host(x) for x in (lo, G, ov)])
+    for a, b in zip(*out):
+        assert np.all(np.isfinite(a.view(float))) and np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("N", [1, 5, 8, 10, 16, 17, 20, 25, 30, 32, 33, 40, 41, 50])
 @pytest.mark.parametrize("fmt", [1, 2])  # TF32, FP16 split
 def test_exchange_tiles(cuda, N, fmt):
