@@ -1031,6 +1031,397 @@ __global__ void __launch_bounds__(PHX_THREADS, sizeof(R) == 4 ? 2 : 1) excited_e
   }
 }
 
+// The same in single precision for eight Cholesky indices per CTA, where their tables fit an SM and no
+// excitation has more than four holes.  Element (row, column) of a table is 64 bytes, the eight
+// indices' complex64 values; four neighbouring lanes hold two indices each, so every table access is
+// a 16-byte load of whole 64-byte runs.
+//   T    [nel][nel + nv]  rows t_j, the reference columns first; Sf takes the virtual columns' place
+//   SU   [nh][nv]
+// Pair p of column c stands at (p + c) & 3 of the run, which spreads the columns of the load from
+// global memory over the banks.  The arithmetic is fma.rn.f32x2 on (re, im) pairs: a complex product
+// is two of them, with one factor's parts doubled and the other's (-im, re).
+// What bound the kernel above is the load-store unit: 32 excitations at their own holes and
+// particles meet in the banks (6.2 cycles for 256 bytes, here 3), their K values went out as 8 bytes
+// to 32 lines at a time (here 64-byte runs), and a table product read five operands for six complex
+// products (here 8 for 32).  512 walkers, 30 + 30 electrons, 20 hole rows, 40 virtual columns, 2220
+// excitations a spin, 960 vectors: 63.1 -> 46.9 ms (load and reference 11, products 14, excitations
+// 22).  What bounds this one is latency: 166 registers and 205 KB leave 12 warps an SM.  512 threads
+// of 128 registers (61.6 ms, spills), two CTAs of four indices (47.1) and one index a lane (66.7) were
+// no faster.
+constexpr int PHG_THREADS = 384;
+constexpr int PHG_N = 8;
+constexpr int PHG_RT = 4, PHG_CT = 4;  // rows and columns of a thread's product tile
+
+using f2 = unsigned long long;  // two packed floats
+__device__ __forceinline__ f2 f2_pack(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// (re, im) -> (-im, re)
+__device__ __forceinline__ f2 f2_i(f2 v) {
+  const float2 x = f2_get(v);
+  return f2_pack(-x.y, x.x);
+}
+__device__ __forceinline__ f2 f2_dup(float a) { return f2_pack(a, a); }
+// o + a b: br, bi the doubled parts of b, ia = i a
+__device__ __forceinline__ f2 f2_cfma(f2 a, f2 ia, f2 br, f2 bi, f2 o) {
+  return f2_fma(ia, bi, f2_fma(a, br, o));
+}
+// two Cholesky indices' values
+struct __align__(16) f2x2 {
+  f2 v[2];
+};
+
+// byte offset of a lane's pair in the run of column c
+__device__ __forceinline__ int phg_slot(int c, int gp) { return ((gp + c) & 3) * 16; }
+
+// the complex64 terms of one excitation for the lane's two indices (excited_terms' sums)
+template <int NEX>
+__device__ __forceinline__ void excited_terms_pair(const int* __restrict__ e4,
+                                                   const c64* __restrict__ Qg, int es,
+                                                   const unsigned char* S, int s_row,
+                                                   const unsigned char* U, int u_row, int gp,
+                                                   const f2 (&f0)[2], f2 (&ex)[2], f2 (&kn)[2]) {
+  c64 Q[NEX * NEX];
+#pragma unroll
+  for (int k = 0; k < NEX * NEX; ++k) Q[k] = Qg[size_t(k) * es];
+  int so[NEX], uo[NEX], pc[NEX];
+#pragma unroll
+  for (int a = 0; a < NEX; ++a) {
+    so[a] = e4[size_t(a) * es] * s_row;
+    uo[a] = e4[size_t(2 * NEX + a) * es] * u_row;
+    const int c = e4[size_t(3 * NEX + a) * es];
+    pc[a] = c * 64 + phg_slot(c, gp);
+  }
+  f2 P[NEX][NEX][2], d[2] = {0ull, 0ull};
+#pragma unroll
+  for (int a = 0; a < NEX; ++a) {
+#pragma unroll
+    for (int b = 0; b < NEX; ++b) P[a][b][0] = P[a][b][1] = 0ull;
+#pragma unroll
+    for (int q = 0; q < NEX; ++q) {
+      const f2x2 s = *reinterpret_cast<const f2x2*>(S + so[a] + pc[q]);
+      const f2x2 u = *reinterpret_cast<const f2x2*>(U + uo[a] + pc[q]);
+      const f2 is[2] = {f2_i(s.v[0]), f2_i(s.v[1])};
+      const c64 qa = Q[a * NEX + q];
+      const f2 qar = f2_dup(qa.x), qai = f2_dup(qa.y);
+#pragma unroll
+      for (int t = 0; t < 2; ++t) d[t] = f2_cfma(u.v[t], f2_i(u.v[t]), qar, qai, d[t]);
+#pragma unroll
+      for (int b = 0; b < NEX; ++b) {
+        const f2 br = f2_dup(Q[b * NEX + q].x), bi = f2_dup(Q[b * NEX + q].y);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) P[a][b][t] = f2_cfma(s.v[t], is[t], br, bi, P[a][b][t]);
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    f2 tr = f0[t], pp = 0ull, off = d[t];
+#pragma unroll
+    for (int a = 0; a < NEX; ++a) {
+      const f2 x = P[a][a][t];
+      const float2 xf = f2_get(x);
+      tr = f2_add(tr, x);
+      pp = f2_cfma(x, f2_i(x), f2_dup(xf.x), f2_dup(xf.y), pp);
+#pragma unroll
+      for (int b = a + 1; b < NEX; ++b) {
+        const float2 y = f2_get(P[b][a][t]);
+        off = f2_cfma(P[a][b][t], f2_i(P[a][b][t]), f2_dup(y.x), f2_dup(y.y), off);
+      }
+    }
+    ex[t] = f2_fma(off, f2_dup(2.f), pp);
+    kn[t] = tr;
+  }
+}
+
+__global__ void __launch_bounds__(PHG_THREADS, 1) excited_energy_groups_kernel(
+    const c64* __restrict__ Twina, const c128* __restrict__ QQ0, const int* __restrict__ refc,
+    const int* __restrict__ hl, const int* __restrict__ vl, int nh, int nv,
+    const int4* __restrict__ uhdr, const int* __restrict__ uexc4, const c64* __restrict__ INVc,
+    int ninv, const c128* __restrict__ wgtT, int nuniq, int W, int nel, int nact, int nchol,
+    c128* __restrict__ EXacc, c128* __restrict__ EJacc, c64* __restrict__ KE,
+    const c64* __restrict__ cross, c128* __restrict__ E, c64* __restrict__ Kref,
+    c128* __restrict__ REF) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int NWARP = PHG_THREADS / 32, NC = PHG_THREADS / 4;
+  const int P = nel + nv, t_row = P * 64, u_row = nv * 64;
+  unsigned char* T = smem_raw;                              // [nel][P] runs
+  unsigned char* SU = T + nel * t_row;                      // [nh][nv] runs
+  float4* Qd = reinterpret_cast<float4*>(SU + nh * u_row);  // [nel][nv] (qr, qr, qi, qi)
+  int* cols = reinterpret_cast<int*>(Qd + nel * nv);        // [P] active columns of T's
+  int* hls = cols + P;                                      // [nh]
+  __shared__ double red[NWARP * 6];
+  __shared__ c128 f0s[PHG_N];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gp = tid & 3, grp = tid >> 2;  // the lane's index pair, its group of four lanes
+  const int n0 = blockIdx.x * PHG_N, w = blockIdx.y;
+  const int ng = min(PHG_N, nchol - n0);
+  const c64* Tw = Twina + size_t(w) * nel * nchol * nact;
+  const c128* Qw = QQ0 + size_t(w) * nact * nel;
+  for (int c = tid; c < P; c += PHG_THREADS) cols[c] = c < nel ? refc[c] : vl[c - nel];
+  for (int k = tid; k < nh; k += PHG_THREADS) hls[k] = hl[k];
+  __syncthreads();
+  // a column's rotation: its place among the reference or the virtual columns
+  for (int r = warp; r < nel * ng; r += NWARP) {
+    const int j = r / ng, g = r - j * ng;
+    const c64* src = Tw + (size_t(j) * nchol + n0 + g) * nact;
+    unsigned char* dst = T + j * t_row + (g & 1) * 8;
+    for (int c = lane; c < P; c += 32)
+      cp_async<8>(dst + c * 64 + phg_slot(c < nel ? c : c - nel, g >> 1), src + cols[c]);
+  }
+  cp_async_commit();
+  for (int k = tid; k < nel * nv; k += PHG_THREADS) {
+    const int i = k / nv, c = k - i * nv;
+    const c64 q = to_cx<c64>(Qw[size_t(vl[c]) * nel + i]);
+    Qd[k] = make_float4(q.x, q.x, q.y, q.y);
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+
+  // the reference determinant: f0 = sum_i t_i[r_i], ex0 = sum_ij t_i[r_j] t_j[r_i]; rows i and
+  // nel - 1 - i together have nel + 1 pairs j >= i
+  auto at = [&](int i, int j) {
+    return *reinterpret_cast<const f2x2*>(T + i * t_row + j * 64 + phg_slot(j, gp));
+  };
+  for (int g = warp; g < ng; g += NWARP) {
+    c128 f = cmk(0, 0);
+    for (int i = lane; i < nel; i += 32)
+      f = cadd(f, to_cx<c128>(*reinterpret_cast<const c64*>(
+                      T + i * t_row + i * 64 + phg_slot(i, g >> 1) + (g & 1) * 8)));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      f.x += __shfl_xor_sync(0xffffffffu, f.x, o);
+      f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
+    }
+    if (lane == 0) {
+      f0s[g] = f;
+      if (Kref) Kref[size_t(w) * nchol + n0 + g] = to_cx<c64>(f);
+    }
+  }
+  c128 ex0 = cmk(0, 0), z1 = cmk(0, 0), z2 = cmk(0, 0);
+  if (Kref)
+    for (int k = grp; k < (nel + 1) / 2 * (nel + 1); k += NC) {
+      const int r = k / (nel + 1), c = k - r * (nel + 1);
+      const bool first = c < nel - r;
+      const int i = first ? r : nel - 1 - r, j = first ? r + c : i + c - (nel - r);
+      if (!first && i == r) continue;  // the middle row stands alone
+      const f2x2 x = at(i, j), y = at(j, i);
+      const double f = i == j ? 1.0 : 2.0;
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+        if (2 * gp + t < ng) {
+          const c128 v = cmul(to_cx<c128>(f2_get(x.v[t])), to_cx<c128>(f2_get(y.v[t])));
+          ex0 = cadd(ex0, cmk(f * v.x, f * v.y));
+        }
+    }
+
+  const int nct = (nv + PHG_CT - 1) / PHG_CT;
+  // Sf = t[:, v] - t[:, r] Qv
+  for (int item = grp; item < (nel + PHG_RT - 1) / PHG_RT * nct; item += NC) {
+    const int rt = item / nct, ct = item - rt * nct;
+    const unsigned char* ar[PHG_RT];
+    int cc[PHG_CT];
+#pragma unroll
+    for (int r = 0; r < PHG_RT; ++r) ar[r] = T + min(rt * PHG_RT + r, nel - 1) * t_row;
+#pragma unroll
+    for (int q = 0; q < PHG_CT; ++q) cc[q] = min(ct + nct * q, nv - 1);
+    f2 acc[PHG_RT][PHG_CT][2];
+#pragma unroll
+    for (int r = 0; r < PHG_RT; ++r)
+#pragma unroll
+      for (int q = 0; q < PHG_CT; ++q) acc[r][q][0] = acc[r][q][1] = 0ull;
+    for (int i = 0; i < nel; ++i) {
+      const int o = i * 64 + phg_slot(i, gp);
+      f2x2 a[PHG_RT];
+      f2 ia[PHG_RT][2];
+#pragma unroll
+      for (int r = 0; r < PHG_RT; ++r) {
+        a[r] = *reinterpret_cast<const f2x2*>(ar[r] + o);
+        ia[r][0] = f2_i(a[r].v[0]);
+        ia[r][1] = f2_i(a[r].v[1]);
+      }
+#pragma unroll
+      for (int q = 0; q < PHG_CT; ++q) {
+        const f2x2 b = *reinterpret_cast<const f2x2*>(Qd + i * nv + cc[q]);
+#pragma unroll
+        for (int r = 0; r < PHG_RT; ++r)
+#pragma unroll
+          for (int t = 0; t < 2; ++t)
+            acc[r][q][t] = f2_cfma(a[r].v[t], ia[r][t], b.v[0], b.v[1], acc[r][q][t]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < PHG_RT; ++r)
+#pragma unroll
+      for (int q = 0; q < PHG_CT; ++q)
+        if (rt * PHG_RT + r < nel && ct + nct * q < nv) {
+          f2x2* x = reinterpret_cast<f2x2*>(T + (rt * PHG_RT + r) * t_row + (nel + cc[q]) * 64 +
+                                            phg_slot(cc[q], gp));
+          f2x2 v = *x;
+#pragma unroll
+          for (int t = 0; t < 2; ++t) v.v[t] = f2_fma(acc[r][q][t], f2_dup(-1.f), v.v[t]);
+          *x = v;
+        }
+  }
+  __syncthreads();
+  // SU = t[hole rows, r] Sf
+  for (int item = grp; item < (nh + PHG_RT - 1) / PHG_RT * nct; item += NC) {
+    const int rt = item / nct, ct = item - rt * nct;
+    const unsigned char* ar[PHG_RT];
+    int bo[PHG_CT];
+#pragma unroll
+    for (int r = 0; r < PHG_RT; ++r) ar[r] = T + hls[min(rt * PHG_RT + r, nh - 1)] * t_row;
+#pragma unroll
+    for (int q = 0; q < PHG_CT; ++q) {
+      const int c = min(ct + nct * q, nv - 1);
+      bo[q] = c * 64 + phg_slot(c, gp);
+    }
+    f2 acc[PHG_RT][PHG_CT][2];
+#pragma unroll
+    for (int r = 0; r < PHG_RT; ++r)
+#pragma unroll
+      for (int q = 0; q < PHG_CT; ++q) acc[r][q][0] = acc[r][q][1] = 0ull;
+    for (int j = 0; j < nel; ++j) {
+      const int o = j * 64 + phg_slot(j, gp);
+      const unsigned char* bj = T + j * t_row + nel * 64;
+      f2x2 b[PHG_CT];
+      f2 ib[PHG_CT][2];
+#pragma unroll
+      for (int q = 0; q < PHG_CT; ++q) {
+        b[q] = *reinterpret_cast<const f2x2*>(bj + bo[q]);
+        ib[q][0] = f2_i(b[q].v[0]);
+        ib[q][1] = f2_i(b[q].v[1]);
+      }
+#pragma unroll
+      for (int r = 0; r < PHG_RT; ++r) {
+        const f2x2 a = *reinterpret_cast<const f2x2*>(ar[r] + o);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const float2 x = f2_get(a.v[t]);
+          const f2 xr = f2_dup(x.x), xi = f2_dup(x.y);
+#pragma unroll
+          for (int q = 0; q < PHG_CT; ++q)
+            acc[r][q][t] = f2_cfma(b[q].v[t], ib[q][t], xr, xi, acc[r][q][t]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < PHG_RT; ++r)
+#pragma unroll
+      for (int q = 0; q < PHG_CT; ++q)
+        if (rt * PHG_RT + r < nh && ct + nct * q < nv) {
+          f2x2 v;
+          v.v[0] = acc[r][q][0];
+          v.v[1] = acc[r][q][1];
+          *reinterpret_cast<f2x2*>(SU + (rt * PHG_RT + r) * u_row + bo[q]) = v;
+        }
+  }
+  __syncthreads();
+
+  c128 f00[2], f00s = cmk(0, 0);
+  f2 f0[2];
+  bool live[2];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    live[t] = 2 * gp + t < ng;
+    const c128 f = live[t] ? f0s[2 * gp + t] : cmk(0, 0);
+    f00[t] = cmul(f, f);
+    f0[t] = f2_pack(float(f.x), float(f.y));
+    if (grp == 0) f00s = cadd(f00s, f00[t]);
+  }
+  block_sum3(ex0, f00s, z2, red);
+  if (tid == 0 && Kref) {
+    atomicAdd(&REF[2 * w].x, ex0.x);
+    atomicAdd(&REF[2 * w].y, ex0.y);
+    atomicAdd(&REF[2 * w + 1].x, f00s.x);
+    atomicAdd(&REF[2 * w + 1].y, f00s.y);
+  }
+  __syncthreads();
+  c128 exs = cmk(0, 0), ejs = cmk(0, 0), ejc = cmk(0, 0);
+  const c64* Iw = INVc + size_t(w) * ninv;
+  const c128* wgw = wgtT + size_t(w) * nuniq;  // this walker's weights, consecutive in u
+  const unsigned char* Sf = T + nel * 64;
+  const bool wide = (nchol & 1) == 0 && live[1];  // 16-byte access to the pair's K
+  int4 hd = 1 + grp < nuniq ? uhdr[1 + grp] : make_int4(0, 0, 0, 0);
+  for (int u = 1 + grp; u < nuniq; u += NC) {
+    const int4 hc = hd;
+    if (u + NC < nuniq) hd = uhdr[u + NC];
+    const c128 wu = wgw[u];
+    const size_t o = (size_t(u) * W + w) * nchol + n0 + 2 * gp;
+    float4 cr = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (cross) {
+      if (wide) {
+        cr = *reinterpret_cast<const float4*>(cross + o);
+      } else {
+        if (live[0]) { cr.x = cross[o].x; cr.y = cross[o].y; }
+        if (live[1]) { cr.z = cross[o + 1].x; cr.w = cross[o + 1].y; }
+      }
+    }
+    const int* e4 = uexc4 + hc.y;
+    const c64* Qi = Iw + hc.z;
+    f2 ex[2], kn[2];
+    switch (hc.x) {
+      case 1: excited_terms_pair<1>(e4, Qi, hc.w, Sf, t_row, SU, u_row, gp, f0, ex, kn); break;
+      case 2: excited_terms_pair<2>(e4, Qi, hc.w, Sf, t_row, SU, u_row, gp, f0, ex, kn); break;
+      case 3: excited_terms_pair<3>(e4, Qi, hc.w, Sf, t_row, SU, u_row, gp, f0, ex, kn); break;
+      default: excited_terms_pair<4>(e4, Qi, hc.w, Sf, t_row, SU, u_row, gp, f0, ex, kn); break;
+    }
+    const float2 k0 = f2_get(kn[0]), k1 = f2_get(kn[1]);
+    if (!cross) {
+      if (wide) {
+        *reinterpret_cast<float4*>(KE + o) = make_float4(k0.x, k0.y, k1.x, k1.y);
+      } else {
+        if (live[0]) KE[o] = k0;
+        if (live[1]) KE[o + 1] = k1;
+      }
+    }
+    c128 exu = cmk(0, 0), eju = cmk(0, 0);
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+      if (live[t]) {
+        const c128 k = to_cx<c128>(t ? k1 : k0);
+        exu = cadd(exu, to_cx<c128>(f2_get(ex[t])));
+        eju = cadd(eju, csub(cmul(k, k), f00[t]));
+        if (cross)
+          ejc = cfma(to_cx<c128>(t ? make_float2(cr.z, cr.w) : make_float2(cr.x, cr.y)), k, ejc);
+      }
+    exs = cfma(wu, exu, exs);
+    ejs = cfma(wu, eju, ejs);
+  }
+  block_sum3(exs, ejs, ejc, red);
+  if (tid == 0) {
+    atomicAdd(&EXacc[w].x, -0.5 * exs.x);
+    atomicAdd(&EXacc[w].y, -0.5 * exs.y);
+    atomicAdd(&EJacc[w].x, 0.5 * ejs.x);
+    atomicAdd(&EJacc[w].y, 0.5 * ejs.y);
+    if (cross) {
+      atomicAdd(&E[w * 3 + 2].x, ejc.x);
+      atomicAdd(&E[w * 3 + 2].y, ejc.y);
+    }
+  }
+}
+
+size_t excited_groups_smem(size_t nel, size_t nh, size_t nv) {
+  return 64 * (nel * (nel + nv) + nh * nv) + 16 * nel * nv + sizeof(int) * (nel + nv + nh);
+}
+
 // The reference determinant's energy from the table sums (ph_reference_kernel's result):
 // E[w] += Ov (E0 + sum_i S[i][r_i], -ex0 / 2, f0^2 / 2)
 __global__ void reference_from_tables_kernel(const c128* __restrict__ Swia,
@@ -2147,7 +2538,16 @@ int phmsd_reference_and_excited(afqmc_phmsd h, cudaStream_t s, int sp, int nb, d
                   : go(excited_energy_tables_kernel<R, 1, TW, false>, tw, inv);
     };
     const c128* twd = h->Twina;
-    if (mixed && h->twina64[sp])
+    const size_t gsm = excited_groups_smem(N, h->nh[sp], h->nv[sp]);
+    if (mixed && h->twina64[sp] && !rare && h->nh[sp] > 0 && gsm <= 225 * 1024) {
+      AFQMC_CUDA_TRY(cudaFuncSetAttribute(excited_energy_groups_kernel,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(gsm)));
+      excited_energy_groups_kernel<<<dim3((Nc + PHG_N - 1) / PHG_N, nb), PHG_THREADS, gsm, s>>>(
+          tw64, h->eQ[sp], h->refc[sp], h->hl[sp], h->vl[sp], h->nh[sp], h->nv[sp], h->uhdrs[sp],
+          h->uexc4s[sp], inv32, h->ninv[sp], h->wgtT, h->nuniq[sp], nb, N, na, Nc, h->el + nb,
+          h->el + 2 * nb, cross ? nullptr : reinterpret_cast<c64*>(KEout),
+          reinterpret_cast<const c64*>(cross), E, reinterpret_cast<c64*>(Kref), REF);
+    } else if (mixed && h->twina64[sp])
       AFQMC_TRY(go_ng(0.f, tw64, inv32));
     else if (mixed)
       AFQMC_TRY(go_ng(0.f, twd, inv32));

@@ -170,3 +170,35 @@ def test_exchange_tiles(cuda, N, fmt):
     E, R = to_host(E), to_host(R)
     for c in (1, 2):
         assert np.max(np.abs(E[:, c] - R[:, c])) < 2e-5 * np.max(np.abs(R[:, c])), c
+
+
+@pytest.mark.parametrize("nup,ndn,nocc,nvirt,Nc,ndet", [(1, 1, 1, 2, 1, 6), (5, 4, 3, 5, 7, 60),
+                                                        (8, 7, 4, 6, 8, 90), (9, 9, 6, 7, 17, 120),
+                                                        (13, 11, 8, 9, 18, 200), (30, 30, 20, 40, 15, 300)])
+def test_phmsd_energy_index_groups(cuda, nup, ndn, nocc, nvirt, Nc, ndet):
+    """The mixed-precision particle-hole energy (groups of eight Cholesky indices, single-precision
+    tables) at remainders of the group, of the product tiles and of the lanes, against complex128.
+    Sums of a few hundred products at 2^-24, amplified by the excitation blocks' inverses: the
+    5e-5 of the comparison with the oracle."""
+    from safire_b200 import afqmc as A
+    from safire_b200.synth import make_hamiltonian, make_phmsd_trial
+    M, W = nup + nvirt + 2, 5
+    M += -M % 8  # the tensor-core rows
+    h1, Likn = make_hamiltonian(M, Nc, 0.9, seed=M)
+    _, C = np.linalg.eigh(h1)
+    t = make_phmsd_trial(M, nup, ndn, C, nocc=nocc, nvirt=nvirt, ndet=ndet, seed=M,
+                         max_level=min(4, 2 * nocc))
+    rs = np.random.default_rng(M + Nc)
+    S = [C[None, :, :n] + rand_c(rs, W, M, n, scale=0.2 / np.sqrt(M)) for n in (nup, ndn)]
+    wbuf = to_dev(np.concatenate([S[0].reshape(W, -1), S[1].reshape(W, -1), np.zeros((W, 11))], 1))
+    ph = A.PHMSD(t)
+    ph.set_hamiltonian(Likn[None], h1[None].astype(complex), 0.3)
+    out = []
+    for prec in (A.PREC_FP64, A.PREC_MIXED):
+        ph.set_precision(prec)
+        E = torch.zeros((W, 3), dtype=torch.complex128, device=cuda)
+        ov = torch.zeros(W, dtype=torch.complex128, device=cuda)
+        ph.Energy(wbuf, E, ov)
+        out.append(to_host(E))
+    scale = np.max(np.abs(out[0]), axis=0)
+    assert np.all(np.abs(out[1] - out[0]) < 5e-5 * scale)
