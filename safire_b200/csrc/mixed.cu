@@ -38,6 +38,7 @@ enum Epi : int {
   EPI_VHS_SYM = 5,   // symmetric L: tile nt = (i block, k block) of the upper triangle; out
                      // planes [row][i][k] and [row][k][i] = split(alpha * acc), alpha real
   EPI_C64T = 6,      // out_c as complex64 [z][col][row] = alpha * col_inv[col] * acc
+  EPI_SUM = 7,       // out_c as complex64 [z][row][col] = acc (n and outc_ld multiples of 4)
 };
 
 // Symmetric vHS tiles: the BN = 128 columns of a tile are the (i, k) pairs of an 8 x 16 block,
@@ -445,6 +446,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_cgemm_kernel(const __grid_co
             vi[j] *= f;
           }
         }
+        if constexpr (EPI == EPI_SUM) {
+          float2* o = reinterpret_cast<float2*>(p.out_c) + long(z) * p.outc_bs +
+                      long(row) * p.outc_ld + n0 + c0;
+#pragma unroll
+          for (int j = 0; j < 16; j += 4)
+            if (n0 + c0 + j < p.n) {
+              uint32_t x[8];
+#pragma unroll
+              for (int t = 0; t < 4; ++t) {
+                x[2 * t] = __float_as_uint(vr[j + t]);
+                x[2 * t + 1] = __float_as_uint(vi[j + t]);
+              }
+              store_sector(o + j, x);
+            }
+          continue;
+        }
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int col = n0 + c0 + j;
@@ -794,6 +811,67 @@ __global__ void __launch_bounds__(SPLIT_ROW_THREADS) split_walkers_T_f16_kernel(
   }
 }
 
+// The same for walkers whose transposed planes fit half an SM's shared memory: coalesced passes over S
+// (the second from L2: the walkers in flight are 47 MB at M = 200, N = 50) and whole lines of the planes'
+// rows, where a thread per row i above reads 16 bytes of a line at a time.
+constexpr int SPLIT_T_THREADS = 1024;
+inline int split_T_pitch(int M) {  // halves: an odd number of words
+  const int w = (M + 1) / 2;
+  return 2 * (w | 1);
+}
+inline size_t split_T_smem(int M, int N) { return size_t(4) * N * split_T_pitch(M) * sizeof(__half); }
+
+__global__ void __launch_bounds__(SPLIT_T_THREADS, 2) split_walkers_T_f16_tile_kernel(
+    const c128* __restrict__ S, long ldS, int M, int N, __half* __restrict__ rh,
+    __half* __restrict__ rl, __half* __restrict__ ih, __half* __restrict__ il, long ld_dst,
+    long bs_dst, float* __restrict__ inv, int pitch) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __half* sm = reinterpret_cast<__half*>(smem_raw);  // [4][N][pitch]
+  __shared__ float wmax[SPLIT_T_THREADS / 32];
+  const long w = blockIdx.x;
+  const c128* Sw = S + w * ldS;
+  const int MN = M * N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float m = 0.f;
+#pragma unroll 4
+  for (int e = threadIdx.x; e < MN; e += SPLIT_T_THREADS) {
+    const c128 v = Sw[e];
+    m = fmaxf(m, fmaxf(fabsf(float(v.x)), fabsf(float(v.y))));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) wmax[warp] = m;
+  __syncthreads();
+  m = 0.f;
+#pragma unroll
+  for (int k = 0; k < SPLIT_T_THREADS / 32; ++k) m = fmaxf(m, wmax[k]);
+  const int ex = tc::f16_scale_exponent(m);
+  const float sc = ldexpf(1.f, ex);
+  if (threadIdx.x == 0) inv[w] = ldexpf(1.f, -ex);
+  const int plane = N * pitch;
+#pragma unroll 4
+  for (int e = threadIdx.x; e < MN; e += SPLIT_T_THREADS) {
+    const c128 v = Sw[e];
+    const int i = e / N, n = e - i * N;
+    __half h, l;
+    tc::f16_split(float(v.x) * sc, h, l);
+    sm[n * pitch + i] = h;
+    sm[plane + n * pitch + i] = l;
+    tc::f16_split(float(v.y) * sc, h, l);
+    sm[2 * plane + n * pitch + i] = h;
+    sm[3 * plane + n * pitch + i] = l;
+  }
+  __syncthreads();
+  for (int r = warp; r < 4 * N; r += SPLIT_T_THREADS / 32) {
+    const int q = r / N, n = r - q * N;
+    __half* dst = (q == 0 ? rh : q == 1 ? rl : q == 2 ? ih : il) + w * bs_dst + long(n) * ld_dst;
+    const __half* src = sm + q * plane + n * pitch;
+    for (int i = 2 * lane; i + 1 < M; i += 64)
+      *reinterpret_cast<uint32_t*>(dst + i) = *reinterpret_cast<const uint32_t*>(src + i);
+    if ((M & 1) && lane == 0) dst[M - 1] = src[M - 1];
+  }
+}
+
+
 // largest |x| of a float64 array (non-negative floats order like their bit patterns)
 __global__ void amax_kernel(const double* __restrict__ x, long n, unsigned* __restrict__ out) {
   float m = 0.f;
@@ -818,13 +896,95 @@ __global__ void split_real_f16_kernel(const double* __restrict__ src, long n_row
   l[d] = lo;
 }
 
+// The same for rows (an even number of columns) that fit the block's registers, 2 KEEP elements a
+// thread: one pass over the source, and stores of two values.  1024 rows of 10000 values: 73 -> 46 us.
+template <int T, int KEEP>
+__global__ void __launch_bounds__(T) split_rows_f16_once_kernel(
+    const c128* __restrict__ src, long ld_src, int cols, __half* __restrict__ rh,
+    __half* __restrict__ rl, __half* __restrict__ ih, __half* __restrict__ il, long ld_dst,
+    float* __restrict__ inv, int rev, float vbound, float* __restrict__ v_inv,
+    float* __restrict__ v_sc) {
+  __shared__ float wmax[T / 32], wsum[T / 32];
+  const long r = blockIdx.x;
+  const c128* row = src + r * ld_src;
+  float4 keep[KEEP];
+  float m = 0.f, l1 = 0.f;
+#pragma unroll
+  for (int k = 0; k < KEEP; ++k) {
+    const int c = 2 * (threadIdx.x + k * T);
+    keep[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < cols) {
+      const c128 a = row[c], b = row[c + 1];
+      keep[k] = make_float4(float(a.x), float(a.y), float(b.x), float(b.y));
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < KEEP; ++k) {
+    const float a = fabsf(keep[k].x), b = fabsf(keep[k].y), c = fabsf(keep[k].z), d = fabsf(keep[k].w);
+    m = fmaxf(m, fmaxf(fmaxf(a, b), fmaxf(c, d)));
+    l1 += (a + b) + (c + d);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    wmax[threadIdx.x >> 5] = m;
+    wsum[threadIdx.x >> 5] = l1;
+  }
+  __syncthreads();
+  m = 0.f;
+  l1 = 0.f;
+#pragma unroll
+  for (int w = 0; w < T / 32; ++w) {
+    m = fmaxf(m, wmax[w]);
+    l1 += wsum[w];
+  }
+  if (v_inv && threadIdx.x == 0) {
+    const int ev = tc::f16_scale_exponent(vbound * l1);
+    v_inv[r] = ldexpf(1.f, -ev);
+    v_sc[r] = ldexpf(1.f, ev);
+  }
+  const int e = tc::f16_scale_exponent(m);
+  const float sc = ldexpf(1.f, e);
+  if (threadIdx.x == 0) inv[r] = ldexpf(1.f, -e);
+#pragma unroll
+  for (int k = 0; k < KEEP; ++k) {
+    const int c = 2 * (threadIdx.x + k * T);
+    if (c >= cols) break;
+    __half2 h, l, hi, li;
+    tc::f16_split(keep[k].x * sc, h.x, l.x);
+    tc::f16_split(keep[k].z * sc, h.y, l.y);
+    tc::f16_split(keep[k].y * sc, hi.x, li.x);
+    tc::f16_split(keep[k].w * sc, hi.y, li.y);
+    long d = r * ld_dst + c;
+    if (rev) {
+      d = r * ld_dst + (cols - 2 - c);
+      h = __lowhigh2highlow(h);
+      l = __lowhigh2highlow(l);
+      hi = __lowhigh2highlow(hi);
+      li = __lowhigh2highlow(li);
+    }
+    *reinterpret_cast<__half2*>(rh + d) = h;
+    *reinterpret_cast<__half2*>(rl + d) = l;
+    *reinterpret_cast<__half2*>(ih + d) = hi;
+    *reinterpret_cast<__half2*>(il + d) = li;
+  }
+}
+
 int split_rows_f16(cudaStream_t s, const c128* src, long ld_src, int rows, int cols, Planes& P,
                    float* inv, bool rev = false, float vbound = 0.f, float* v_inv = nullptr,
                    float* v_sc = nullptr) {
-  split_rows_f16_kernel<<<rows, SPLIT_ROW_THREADS, 0, s>>>(src, ld_src, cols, P.h(0), P.h(1),
-                                                           P.h(2), P.h(3), P.ld, inv,
-                                                           rev ? 1 : 0, vbound, v_inv, v_sc);
-  return launch_status("split_rows_f16_kernel");
+  auto go = [&](auto kern, int threads) -> int {
+    kern<<<rows, threads, 0, s>>>(src, ld_src, cols, P.h(0), P.h(1), P.h(2), P.h(3), P.ld, inv,
+                                  rev ? 1 : 0, vbound, v_inv, v_sc);
+    return launch_status("split_rows_f16_kernel");
+  };
+  // rows start on 16 bytes, so pairs of halves are aligned
+  if (cols % 2 == 0 && cols <= 2 * 4 * 256) return go(split_rows_f16_once_kernel<256, 4>, 256);
+  if (cols % 2 == 0 && cols <= 2 * 8 * 1024) return go(split_rows_f16_once_kernel<1024, 8>, 1024);
+  return go(split_rows_f16_kernel, SPLIT_ROW_THREADS);
 }
 
 // static real tensor [rows][cols] (device, synchronous set-up): one scale for the whole tensor;
@@ -931,7 +1091,7 @@ struct MixedHam {
   int taylor_one_slot = 0;  // 0 second accumulator, 1 running sum in tensor memory
   Planes G;         // [W][1][nel_tot*M]  (A of vbias);  exchange view [W*nel][M]
   Planes X;         // [1][W][Nc] (A of vHS)
-  c128* vpart = nullptr;  // split-K partial sums of vbias [S][W][Nc]
+  float2* vpart = nullptr;  // split-K partial sums of vbias [S][W][Nc]
   long vpart_elems = 0;
   unsigned* err = nullptr;
   // propagation buffers
@@ -1114,14 +1274,31 @@ int ensure_walker_buffers(MixedHam* m, int W) {
 }  // namespace
 
 namespace {
-// v[i] (+)= sum_s part[s][i] in FP64
-__global__ void sum_partials_kernel(const c128* __restrict__ part, int S, long n,
+// v[i] (+)= alpha sum_s part[s][i] in FP64, two elements a thread.  part: the accumulators themselves
+// in complex64 (EPI_SUM); scaled to complex128 by the GEMM they were twice the bytes, in 16-byte pieces
+// to 32 rows at a time: 283 + 51 us for 1024 walkers of 10000 values, 1600 vectors, ten ranges, now 209
+// + 27.
+__global__ void sum_partials_kernel(const float4* __restrict__ part, int S, long n2, c128 alpha,
                                     c128* __restrict__ v, int accumulate) {
   const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  c128 acc = accumulate ? v[i] : cmk(0, 0);
-  for (int z = 0; z < S; ++z) acc = cadd(acc, part[long(z) * n + i]);
-  v[i] = acc;
+  if (i >= n2) return;
+  c128 a = cmk(0, 0), b = cmk(0, 0);
+#pragma unroll 4
+  for (int z = 0; z < S; ++z) {
+    const float4 x = part[long(z) * n2 + i];
+    a = cadd(a, cmk(x.x, x.y));
+    b = cadd(b, cmk(x.z, x.w));
+  }
+  a = cmul(alpha, a);
+  b = cmul(alpha, b);
+  v[2 * i] = accumulate ? cadd(v[2 * i], a) : a;
+  v[2 * i + 1] = accumulate ? cadd(v[2 * i + 1], b) : b;
+}
+
+int sum_partials(cudaStream_t s, MixedHam* m, int S, long n, c128 alpha, c128* v, bool accumulate) {
+  sum_partials_kernel<<<ceil_div(n / 2, 256), 256, 0, s>>>(
+      reinterpret_cast<const float4*>(m->vpart), S, n / 2, alpha, v, accumulate ? 1 : 0);
+  return launch_status("sum_partials_kernel");
 }
 }  // namespace
 
@@ -1143,17 +1320,15 @@ int vbias_mixed_f16(cudaStream_t s, MixedHam* m, const c128* G, long ldG, c128* 
     }
   TcParams p{};
   const long Kc = K / S;
-  c128* out = v;
   if (S > 1) {
     const long need = long(S) * W * m->Nc;
     if (m->vpart_elems < need) {
       if (m->vpart) cudaFree(m->vpart);
       m->vpart = nullptr;
       m->vpart_elems = 0;
-      AFQMC_CUDA_TRY(cudaMalloc(&m->vpart, sizeof(c128) * need));
+      AFQMC_CUDA_TRY(cudaMalloc(&m->vpart, sizeof(float2) * need));
       m->vpart_elems = need;
     }
-    out = m->vpart;
   }
   for (int q = 0; q < 4; ++q)
     AFQMC_TRY(make_map_es(&p.a[q], m->G16, q, 0, Kc, W, m->G16.ld, S, Kc, 128));
@@ -1165,18 +1340,18 @@ int vbias_mixed_f16(cudaStream_t s, MixedHam* m, const c128* G, long ldG, c128* 
   p.order = 1;
   p.alpha = cmk(a * double(m->lnak_inv), 0);
   p.row_inv = m->g_inv;
-  p.out_c = out; p.outc_ld = m->Nc; p.outc_bs = long(W) * m->Nc;
+  p.out_c = S > 1 ? reinterpret_cast<c128*>(m->vpart) : v;
+  p.outc_ld = m->Nc; p.outc_bs = long(W) * m->Nc;
   p.err = m->err;
-  if (bn == 64)
-    AFQMC_TRY((launch_tc<true, false, 64, 2, EPI_C128, true>(s, p, S)));
-  else
-    AFQMC_TRY((launch_tc<true, false, 128, 2, EPI_C128, true>(s, p, S)));
-  if (S > 1) {
-    const long n = long(W) * m->Nc;
-    sum_partials_kernel<<<ceil_div(n, 256), 256, 0, s>>>(m->vpart, S, n, v, 0);
-    AFQMC_TRY(launch_status("sum_partials_kernel"));
+  if (S == 1) {
+    if (bn == 64) return launch_tc<true, false, 64, 2, EPI_C128, true>(s, p, S);
+    return launch_tc<true, false, 128, 2, EPI_C128, true>(s, p, S);
   }
-  return AFQMC_OK;
+  if (bn == 64)
+    AFQMC_TRY((launch_tc<true, false, 64, 2, EPI_SUM, true>(s, p, S)));
+  else
+    AFQMC_TRY((launch_tc<true, false, 128, 2, EPI_SUM, true>(s, p, S)));
+  return sum_partials(s, m, S, long(W) * m->Nc, p.alpha, v, false);
 }
 }  // namespace
 
@@ -1215,7 +1390,7 @@ int vbias_mixed(cudaStream_t s, MixedHam* m, const c128* G, long ldG, c128* v, i
         if (m->vpart) cudaFree(m->vpart);
         m->vpart = nullptr;
         m->vpart_elems = 0;
-        AFQMC_CUDA_TRY(cudaMalloc(&m->vpart, sizeof(c128) * need));
+        AFQMC_CUDA_TRY(cudaMalloc(&m->vpart, sizeof(float2) * need));
         m->vpart_elems = need;
       }
       // 3-D maps whose third coordinate steps through the K ranges (stride Kc floats)
@@ -1230,12 +1405,10 @@ int vbias_mixed(cudaStream_t s, MixedHam* m, const c128* G, long ldG, c128* v, i
         p.a_batched = 1; p.b_batched = 1;
         p.order = 1;
         p.alpha = cmk(a, 0);
-        p.out_c = m->vpart; p.outc_ld = m->Nc; p.outc_bs = long(W) * m->Nc;
+        p.out_c = reinterpret_cast<c128*>(m->vpart); p.outc_ld = m->Nc; p.outc_bs = long(W) * m->Nc;
         p.err = m->err;
-        AFQMC_TRY((launch_tc<true, false, 128, 2, EPI_C128>(s, p, S)));
-        const long n = long(W) * m->Nc;
-        sum_partials_kernel<<<ceil_div(n, 256), 256, 0, s>>>(m->vpart, S, n, v, first ? 0 : 1);
-        AFQMC_TRY(launch_status("sum_partials_kernel"));
+        AFQMC_TRY((launch_tc<true, false, 128, 2, EPI_SUM>(s, p, S)));
+        AFQMC_TRY(sum_partials(s, m, S, long(W) * m->Nc, p.alpha, v, !first));
       }
     }
     if (!split) {
@@ -1471,9 +1644,18 @@ int propagate_mixed(cudaStream_t s, MixedHam* m, const void* P1, bool p1_real, c
                                     &m->p1_inv));
       m->P1_16_src = P1;
     }
-    split_walkers_T_f16_kernel<<<W, SPLIT_ROW_THREADS, 0, s>>>(
-        S, ldS, M, N, m->Sst16.h(0), m->Sst16.h(1), m->Sst16.h(2), m->Sst16.h(3), m->Sst16.ld,
-        m->Sst16.bstride(), m->s_inv);
+    const size_t tsm = split_T_smem(M, N);
+    if (tsm <= 110 * 1024) {
+      AFQMC_CUDA_TRY(cudaFuncSetAttribute(split_walkers_T_f16_tile_kernel,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(tsm)));
+      split_walkers_T_f16_tile_kernel<<<W, SPLIT_T_THREADS, tsm, s>>>(
+          S, ldS, M, N, m->Sst16.h(0), m->Sst16.h(1), m->Sst16.h(2), m->Sst16.h(3), m->Sst16.ld,
+          m->Sst16.bstride(), m->s_inv, split_T_pitch(M));
+    } else {
+      split_walkers_T_f16_kernel<<<W, SPLIT_ROW_THREADS, 0, s>>>(
+          S, ldS, M, N, m->Sst16.h(0), m->Sst16.h(1), m->Sst16.h(2), m->Sst16.h(3), m->Sst16.ld,
+          m->Sst16.bstride(), m->s_inv);
+    }
     AFQMC_TRY(launch_status("split_walkers_T_f16_kernel"));
     const void* p1p[2] = {m->P1_16.p[0], m->P1_16.p[1]};
     const void* vp[4] = {m->V16.p[0], m->V16.p[1], m->V16.p[2], m->V16.p[3]};

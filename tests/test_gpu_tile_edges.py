@@ -202,3 +202,26 @@ def test_phmsd_energy_index_groups(cuda, nup, ndn, nocc, nvirt, Nc, ndet):
         out.append(to_host(E))
     scale = np.max(np.abs(out[0]), axis=0)
     assert np.all(np.abs(out[1] - out[0]) < 5e-5 * scale)
+
+
+@pytest.mark.parametrize("M,N,Nc,W", [(40, 13, 8, 1), (72, 32, 44, 130), (104, 50, 264, 33), (136, 50, 24, 7)])
+@pytest.mark.parametrize("fmt", [1, 2])  # TF32, FP16 split
+def test_mixed_vbias_ranges(cuda, M, N, Nc, W, fmt):
+    """The force bias summed over ranges of its K = N M (one, and several) in mixed precision, against
+    complex128.  Operands keep 22 bits, and a running sum in FP32 loses up to 2^-23 of itself with
+    each MMA of 16 elements; it is about the size of a result, of which the largest of the deviations
+    is taken as eight."""
+    from safire_b200 import afqmc as A
+    rs = np.random.default_rng(M)
+    Nc -= Nc % 8 if fmt == 2 else 0  # the FP16 split takes multiples of 8
+    L = rs.standard_normal((M, M, Nc))
+    ham = _ham(M, N, Nc, L + L.transpose(1, 0, 2))
+    ham.set_split_format(fmt)
+    G = to_dev(rand_c(rs, W, N * M))
+    v, r = (torch.empty((W, Nc), dtype=torch.complex128, device=cuda) for _ in range(2))
+    ham.vbias(G, v, 0.01, precision=A.PREC_MIXED)
+    ham.vbias(G, r, 0.01)
+    assert ham.device_error_flag() == 0
+    v, r = to_host(v), to_host(r)
+    bound = 8 * (2.0 ** -21 + N * M / 16 * 2.0 ** -23)
+    assert np.max(np.abs(v - r)) < bound * np.sqrt(np.mean(np.abs(r) ** 2))
