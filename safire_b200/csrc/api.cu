@@ -1230,43 +1230,77 @@ int nomsd_bufs(afqmc_nomsd md, int W) {
   return AFQMC_OK;
 }
 
+// The sums over a walker's determinants below: one warp per walker, the determinants over its lanes.
+// A thread per walker was a chain of ndet complex exponentials on a dozen CTAs: 21 and 28 us for
+// 1536 walkers of 34 determinants, now 5 and 4.
+constexpr int WD_WARPS = 4;
+
+__device__ __forceinline__ c128 warp_sum(c128 x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    x.x += __shfl_xor_sync(0xffffffffu, x.x, o);
+    x.y += __shfl_xor_sync(0xffffffffu, x.y, o);
+  }
+  return x;
+}
+
 // out[w] = m + log sum_d exp(ovd[w][d] + lc[d] - m), m = the largest real part of the
-// ovd[w][d] + lc[d] (NOMSD.cpp:303-331: per-determinant log overlap + log conj(ci))
-__global__ void logsumexp_wd_kernel(const c128* __restrict__ ovd, const c128* __restrict__ lc,
-                                    int ndet, int W, c128* __restrict__ out) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+// ovd[w][d] + lc[d], the first of equal ones (NOMSD.cpp:303-331: per-determinant log overlap +
+// log conj(ci))
+__global__ void __launch_bounds__(32 * WD_WARPS)
+    logsumexp_wd_kernel(const c128* __restrict__ ovd, const c128* __restrict__ lc, int ndet, int W,
+                        c128* __restrict__ out) {
+  const int w = blockIdx.x * WD_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (w >= W) return;
   const c128* o = ovd + size_t(w) * ndet;
-  c128 m = cadd(o[0], lc[0]);
-  for (int d = 1; d < ndet; ++d) {
-    const c128 x = cadd(o[d], lc[d]);
-    if (x.x > m.x) m = x;
+  int at = -1;  // this lane's largest
+  double best = 0.0;
+  for (int d = lane; d < ndet; d += 32) {
+    const double x = o[d].x + lc[d].x;
+    if (at < 0 || x > best) {
+      best = x;
+      at = d;
+    }
   }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const double ob = __shfl_xor_sync(0xffffffffu, best, s);
+    const int oa = __shfl_xor_sync(0xffffffffu, at, s);
+    if (oa >= 0 && (at < 0 || ob > best || (ob == best && oa < at))) {
+      best = ob;
+      at = oa;
+    }
+  }
+  at = __shfl_sync(0xffffffffu, at, 0);  // one choice also where comparisons meet NaNs
+  const c128 m = cadd(o[at], lc[at]);
   c128 sum = cmk(0, 0);
-  for (int d = 0; d < ndet; ++d) sum = cadd(sum, cexp(csub(cadd(o[d], lc[d]), m)));
-  out[w] = cadd(m, clog(sum));
+  for (int d = lane; d < ndet; d += 32) sum = cadd(sum, cexp(csub(cadd(o[d], lc[d]), m)));
+  sum = warp_sum(sum);
+  if (lane == 0) out[w] = cadd(m, clog(sum));
 }
 
 // f_d = conj(c_d) exp(ovd[w][d] - ovlp_w) with ovlp_w the walker's stored log overlap;
 // wdd[w][d] = f_d / sum_d f_d, Ov[w] = sum_d f_d + ovlp_w (NOMSD.cpp:220-279: the reference
 // divides the summed G by the linear sum and then adds the log of the shift to it)
-__global__ void multidet_weights_kernel(const c128* __restrict__ ovd, const c128* __restrict__ cc,
-                                        int ndet, int W, const c128* __restrict__ wbuf, long ldw,
-                                        long prop_ovlp, c128* __restrict__ wdd,
-                                        c128* __restrict__ Ov) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * WD_WARPS)
+    multidet_weights_kernel(const c128* __restrict__ ovd, const c128* __restrict__ cc, int ndet,
+                            int W, const c128* __restrict__ wbuf, long ldw, long prop_ovlp,
+                            c128* __restrict__ wdd, c128* __restrict__ Ov) {
+  const int w = blockIdx.x * WD_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (w >= W) return;
   const c128 shift = wbuf[long(w) * ldw + prop_ovlp];
   const c128* o = ovd + size_t(w) * ndet;
   c128* f = wdd + size_t(w) * ndet;
   c128 sum = cmk(0, 0);
-  for (int d = 0; d < ndet; ++d) {
-    f[d] = cmul(cc[d], cexp(csub(o[d], shift)));
-    sum = cadd(sum, f[d]);
+  for (int d = lane; d < ndet; d += 32) {
+    const c128 x = cmul(cc[d], cexp(csub(o[d], shift)));
+    f[d] = x;
+    sum = cadd(sum, x);
   }
+  sum = warp_sum(sum);
   const c128 inv = cdiv(cmk(1, 0), sum);
-  for (int d = 0; d < ndet; ++d) f[d] = cmul(f[d], inv);
-  Ov[w] = cadd(sum, shift);
+  for (int d = lane; d < ndet; d += 32) f[d] = cmul(f[d], inv);
+  if (lane == 0) Ov[w] = cadd(sum, shift);
 }
 
 // Tt[b] = wdd[b] T[b]^T for nb blocks of n x n elements
@@ -1317,7 +1351,7 @@ int nomsd_log_overlap(afqmc_nomsd md, afqmc_wset_s* ws, cudaStream_t s, c128* ov
   for (int w0 = 0; w0 < W; w0 += md->wchunk) {
     const int wc = std::min(md->wchunk, W - w0);
     AFQMC_TRY(nomsd_overlaps(md, ws, s, w0, wc, false));
-    logsumexp_wd_kernel<<<ceil_div(wc, 128), 128, 0, s>>>(md->ovd, md->dlc, nd, wc, ovlp + w0);
+    logsumexp_wd_kernel<<<ceil_div(wc, WD_WARPS), 32 * WD_WARPS, 0, s>>>(md->ovd, md->dlc, nd, wc, ovlp + w0);
     AFQMC_TRY(launch_status("logsumexp_wd_kernel"));
   }
   return AFQMC_OK;
@@ -1337,7 +1371,7 @@ int nomsd_density_matrix(afqmc_nomsd md, afqmc_wset_s* ws, cudaStream_t s, c128*
     const c128* S0 = ws->buf + long(w0) * ws->walker_size;
     c128* Gw = G + long(w0) * per;
     AFQMC_TRY(nomsd_overlaps(md, ws, s, w0, wc, true));
-    multidet_weights_kernel<<<ceil_div(wc, 128), 128, 0, s>>>(
+    multidet_weights_kernel<<<ceil_div(wc, WD_WARPS), 32 * WD_WARPS, 0, s>>>(
         md->ovd, md->dcc, nd, wc, S0, ws->walker_size, ws->prop0 + AFQMC_OVLP, md->wdd, Ov + w0);
     AFQMC_TRY(launch_status("multidet_weights_kernel"));
     long toff = 0;

@@ -149,6 +149,35 @@ def test_real_trial(cuda, M, N, W, ndet):
         assert np.all(np.isfinite(a.view(float))) and np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("ndet,W", [(2, 1), (31, 5), (32, 3), (33, 9), (70, 4)])
+def test_determinant_sums(cuda, ndet, W):
+    """Log overlap and density matrix of several determinants at the lanes' remainders, against
+    numpy: the sums are weighted means, so eps times their length and the conditions of the
+    overlap matrices bounds the error."""
+    from safire_b200 import afqmc as A
+    M, N = 7, 2
+    rs = np.random.default_rng(ndet)
+    psi = rs.standard_normal((ndet, N, M))
+    S = np.eye(M, N) + rand_c(rs, W, M, N, scale=0.3)
+    ci = rs.uniform(0.1, 1.0, ndet)
+    L, hij = np.zeros((M, M, 2)), np.eye(M)[None].astype(complex)
+    hams = [A.HamiltonianOperations(A.CLOSED, M, N, N, L[None], hij, 0.0, [p.astype(complex)])
+            for p in psi]
+    wset = A.WalkerSet(A.CLOSED, M, N, N, W)
+    wset.init_from_trial(hams[0])
+    wset.SlaterMatrices(0).copy_(to_dev(S))
+    md = A.NOMSDMulti(hams, ci.astype(complex))
+    T = np.einsum("dai,wib->wdab", psi, S)
+    f = ci * np.linalg.det(T) ** 2
+    cond = np.max(np.linalg.cond(T)) * np.max(np.sum(np.abs(f), 1) / np.abs(np.sum(f, 1)))
+    lo = to_host(md.Log_Overlap(wset))
+    assert np.max(np.abs(np.exp(lo - np.log(np.sum(f, 1))) - 1)) < 50 * ndet * EPS * cond
+    G = to_host(md.MixedDensityMatrix(wset)[0]).reshape(W, M, M)
+    Gd = np.einsum("dai,wdba,wkb->wdik", psi, np.linalg.inv(T), S)
+    want = np.einsum("wd,wdik->wik", f / np.sum(f, 1, keepdims=True), Gd)
+    assert np.max(np.abs(G - want)) < 50 * ndet * EPS * cond * np.max(np.abs(Gd))
+
+
 @pytest.mark.parametrize("N", [1, 5, 8, 10, 16, 17, 20, 25, 30, 32, 33, 40, 41, 50])
 @pytest.mark.parametrize("fmt", [1, 2])  # TF32, FP16 split
 def test_exchange_tiles(cuda, N, fmt):
