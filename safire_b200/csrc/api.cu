@@ -141,6 +141,7 @@ struct afqmc_prop_s {
   int nspin_P1 = 1, nspin_V = 1;
   c128* P1 = nullptr;        // [nspin][M][M]
   double* P1r = nullptr;     // real copy when real
+  MixedP1* P1_mixed[2] = {nullptr, nullptr};  // its split planes per spin (mixed steps)
   c128* vMF = nullptr;       // [Nc]
   std::vector<c128> P1_h, vMF_h;
   double mf0 = 0;            // -Re(vMF.vMF)/2
@@ -161,11 +162,20 @@ struct afqmc_prop_s {
   // per-phase CUDA events of the last timed step (AFQMCTimers analogue)
   bool timing = false;
   cudaEvent_t ev[AFQMC_NPHASE + 1] = {};
+  // P1 and what was made from it
+  void free_P1() {
+    dfree(P1); dfree(P1r);
+    for (auto& q : P1_mixed) {
+      if (q) mixed_p1_destroy(q);
+      q = nullptr;
+    }
+  }
   ~afqmc_prop_s() {
     DeviceGuard g(device);
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
-    dfree(P1); dfree(P1r); dfree(vMF);
+    free_P1();
+    dfree(vMF);
     dfree(G); dfree(vb); dfree(X); dfree(HW); dfree(mf); dfree(newov); dfree(ovtmp);
     dfree(T); dfree(V); dfree(w1); dfree(w2); dfree(w3); dfree(ortho_work);
     dfree(Eshift_d); dfree(counter); dfree(stats); dfree(Gph); dfree(Gfull);
@@ -1758,8 +1768,7 @@ static int prop_mean_field(afqmc_prop_s* pr, const c128* vMF_host) {
   pr->p1_real = real;
   pr->nspin_P1 = nspin;
   pr->nspin_V = h->walker_type == AFQMC_COLLINEAR ? h->nspin_H2 : 1;
-  dfree(pr->P1);
-  dfree(pr->P1r);
+  pr->free_P1();
   dfree(pr->vMF);
   AFQMC_TRY(dalloc(&pr->P1, size_t(nspin) * MM));
   AFQMC_CUDA_TRY(cudaMemcpy(pr->P1, pr->P1_h.data(), sizeof(c128) * nspin * MM,
@@ -1976,8 +1985,9 @@ int prop_step(afqmc_prop_s* pr, afqmc_wset_s* ws, double Eshift, const double* E
                                  : (const void*)(pr->P1 + size_t(sp % pr->nspin_P1) * MM);
     const c128* V = pr->V + size_t(sp % pr->nspin_V) * W * MM;
     if (mixed) {
-      AFQMC_TRY(propagate_mixed(s, h->mixed, P1, pr->p1_real, ws->buf + ws->offS(sp),
-                                ws->walker_size, W, M, Ns, pr->p.taylor_n));
+      AFQMC_TRY(propagate_mixed(s, h->mixed, &pr->P1_mixed[sp % pr->nspin_P1], P1, pr->p1_real,
+                                ws->buf + ws->offS(sp), ws->walker_size, W, M, Ns,
+                                pr->p.taylor_n));
     } else {
       AFQMC_TRY(propagate(s, P1, pr->p1_real, V, MM, ws->buf + ws->offS(sp), ws->walker_size, W, M,
                           Ns, pr->p.taylor_n, pr->w1, pr->w2, pr->w3));

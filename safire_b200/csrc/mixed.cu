@@ -13,8 +13,8 @@
 
 #include <cstring>
 #include <memory>
-#include <new>
 #include <mutex>
+#include <new>
 
 #include "detops.cuh"
 #include "energy.cuh"
@@ -1072,13 +1072,11 @@ struct MixedHam {
   int capW16 = 0;
   float likn_amax = 0.f;   // largest |L| (bound of V's scale)
   // FP16 propagation: V planes [W][M][M] with per-walker scales (from a * sum_n |X_n| max |L|),
-  // P1 planes, S^T / T / R planes [W][N][M]
-  Planes V16, P1_16, Sst16, T0_16, T1_16, R16;
+  // S^T / T / R planes [W][N][M]
+  Planes V16, Sst16, T0_16, T1_16, R16;
   float* v_inv = nullptr;  // [W]
   float* v_sc = nullptr;   // [W]
   float* s_inv = nullptr;  // [W]
-  float p1_inv = 1.f;
-  const void* P1_16_src = nullptr;
   int capP16 = 0;
   bool v_is_f16 = false;   // format of the V planes the last vHS wrote
   // Taylor propagation (mixed_set_taylor_mode): 0 one GEMM launch per product; 2 / 3 the fused
@@ -1096,8 +1094,6 @@ struct MixedHam {
   unsigned* err = nullptr;
   // propagation buffers
   int capP = 0;
-  Planes P1;        // [1][M][M] real (A of the P1 products)
-  const void* P1_src = nullptr;
   Planes V;         // [W][M][M] complex (A of the Taylor products)
   Planes T0, T1, Tacc_split, Sst;  // [W][N][M] complex (B operands)
   float* acc[2] = {nullptr, nullptr};  // running Taylor sum [W][N][M]
@@ -1115,7 +1111,6 @@ struct MixedHam {
     if (g_inv) cudaFree(g_inv);
     if (x_inv) cudaFree(x_inv);
     free_planes(V16);
-    free_planes(P1_16);
     free_planes(Sst16);
     free_planes(T0_16);
     free_planes(T1_16);
@@ -1123,7 +1118,6 @@ struct MixedHam {
     if (v_inv) cudaFree(v_inv);
     if (v_sc) cudaFree(v_sc);
     if (s_inv) cudaFree(s_inv);
-    free_planes(P1);
     free_planes(V);
     free_planes(T0);
     free_planes(T1);
@@ -1137,6 +1131,20 @@ struct MixedHam {
 };
 
 void mixed_ham_destroy(MixedHam* m) { delete m; }
+
+// One-body propagator of one spin block, real [M][M] (A of the P1 products), in the format of the V
+// planes that it meets.  They live as long as the P1 that they were split from: its propagator owns
+// them, so that another propagator of the Hamiltonian, or another mean field, brings its own.
+struct MixedP1 {
+  Planes tf32, f16;
+  float f16_inv = 1.f;  // inverse scale of f16
+  ~MixedP1() {
+    free_planes(tf32);
+    free_planes(f16);
+  }
+};
+
+void mixed_p1_destroy(MixedP1* p) { delete p; }
 
 namespace {
 // max |L[i][k][n] - L[k][i][n]| and max |L| (as ordered bit patterns of non-negative doubles)
@@ -1620,8 +1628,8 @@ int taylor_fused_tc(cudaStream_t s, int esize, const void* const P1p[2], const v
 
 // Taylor propagation S <- P1 sum_n (iV)^n/n! P1 S (propagate.hpp:238-298) on the split planes.
 // V must have been produced by vhs_mixed (planes kept in MixedHam) for the same walkers.
-int propagate_mixed(cudaStream_t s, MixedHam* m, const void* P1, bool p1_real, c128* S, long ldS,
-                    int W, int M, int N, int order) {
+int propagate_mixed(cudaStream_t s, MixedHam* m, MixedP1** planes, const void* P1, bool p1_real,
+                    c128* S, long ldS, int W, int M, int N, int order) {
   if (!p1_real) {
     set_error_detail("propagate_mixed: a complex one-body propagator is not supported");
     return AFQMC_ERR_UNSUPPORTED;
@@ -1631,18 +1639,24 @@ int propagate_mixed(cudaStream_t s, MixedHam* m, const void* P1, bool p1_real, c
     return AFQMC_ERR_ARG;
   }
   AFQMC_TRY(ensure_prop_buffers(m, W, N));
+  if (!*planes) *planes = new (std::nothrow) MixedP1();
+  AFQMC_CHECK_ARG(*planes, "propagate_mixed: out of host memory");
+  MixedP1& p1 = **planes;
   if (m->v_is_f16) {
     if (M > 256 || N > 64) {
       set_error_detail("propagate_mixed: FP16 V planes need M <= 256 and N <= 64");
       return AFQMC_ERR_UNSUPPORTED;
     }
     AFQMC_TRY(ensure_prop_buffers16(m, W, N));
-    if (m->P1_16_src != P1) {
-      free_planes(m->P1_16);
-      AFQMC_TRY(alloc_planes(m->P1_16, 2, 1, M, M, 2));
-      AFQMC_TRY(split_real_f16_host(static_cast<const double*>(P1), M, M, M, m->P1_16,
-                                    &m->p1_inv));
-      m->P1_16_src = P1;
+    if (!p1.f16.p[0]) {
+      Planes f16;
+      int st = alloc_planes(f16, 2, 1, M, M, 2);
+      if (!st) st = split_real_f16_host(static_cast<const double*>(P1), M, M, M, f16, &p1.f16_inv);
+      if (st) {
+        free_planes(f16);
+        return st;
+      }
+      p1.f16 = f16;
     }
     const size_t tsm = split_T_smem(M, N);
     if (tsm <= 110 * 1024) {
@@ -1657,31 +1671,35 @@ int propagate_mixed(cudaStream_t s, MixedHam* m, const void* P1, bool p1_real, c
           m->Sst16.bstride(), m->s_inv);
     }
     AFQMC_TRY(launch_status("split_walkers_T_f16_kernel"));
-    const void* p1p[2] = {m->P1_16.p[0], m->P1_16.p[1]};
+    const void* p1p[2] = {p1.f16.p[0], p1.f16.p[1]};
     const void* vp[4] = {m->V16.p[0], m->V16.p[1], m->V16.p[2], m->V16.p[3]};
     const void* sp[4] = {m->Sst16.p[0], m->Sst16.p[1], m->Sst16.p[2], m->Sst16.p[3]};
     void* t0[4] = {m->T0_16.p[0], m->T0_16.p[1], m->T0_16.p[2], m->T0_16.p[3]};
     void* t1[4] = {m->T1_16.p[0], m->T1_16.p[1], m->T1_16.p[2], m->T1_16.p[3]};
     void* rp[4] = {m->R16.p[0], m->R16.p[1], m->R16.p[2], m->R16.p[3]};
-    if (m->P1_16.ld != m->T0_16.ld || m->T0.ld != m->T0_16.ld) {
+    if (p1.f16.ld != m->T0_16.ld || m->T0.ld != m->T0_16.ld) {
       set_error_detail("propagate_mixed: FP16 plane strides differ (M = %d)", M);
       return AFQMC_ERR_UNSUPPORTED;
     }
     return taylor_fused_tc(s, 2, p1p, vp, m->V16.ld, sp, t0, t1, rp, m->acc, m->T0_16.ld, S, ldS,
                            W, M, N, order, m->taylor_slots, m->taylor_one_slot, m->v_inv,
-                           m->s_inv, m->p1_inv, m->err);
+                           m->s_inv, p1.f16_inv, m->err);
   }
-  if (m->P1_src != P1) {
-    free_planes(m->P1);
-    AFQMC_TRY(alloc_planes(m->P1, 2, 1, M, M));
-    AFQMC_TRY(split_real_host(static_cast<const double*>(P1), M, M, M, m->P1));
-    m->P1_src = P1;
+  if (!p1.tf32.p[0]) {
+    Planes tf32;
+    int st = alloc_planes(tf32, 2, 1, M, M);
+    if (!st) st = split_real_host(static_cast<const double*>(P1), M, M, M, tf32);
+    if (st) {
+      free_planes(tf32);
+      return st;
+    }
+    p1.tf32 = tf32;
   }
   // S^T planes [W][N][M] from the walkers' Slater matrices [W][M][N]
   AFQMC_TRY(split_complex(s, S, N, ldS, W, M, N, m->Sst, true));
-  if (M <= 256 && N <= 64 && m->taylor_mode != 0 && m->P1.ld == m->T0.ld) {
+  if (M <= 256 && N <= 64 && m->taylor_mode != 0 && p1.tf32.ld == m->T0.ld) {
     // one persistent kernel runs all order + 2 products of each walker
-    const void* p1p[2] = {m->P1.p[0], m->P1.p[1]};
+    const void* p1p[2] = {p1.tf32.p[0], p1.tf32.p[1]};
     const void* vp[4] = {m->V.p[0], m->V.p[1], m->V.p[2], m->V.p[3]};
     const void* sp[4] = {m->Sst.p[0], m->Sst.p[1], m->Sst.p[2], m->Sst.p[3]};
     void* t0[4] = {m->T0.p[0], m->T0.p[1], m->T0.p[2], m->T0.p[3]};
@@ -1697,7 +1715,7 @@ int propagate_mixed(cudaStream_t s, MixedHam* m, const void* P1, bool p1_real, c
   // T0 = P1 S  (acc = T0)
   {
     TcParams p{};
-    AFQMC_TRY(maps_for(m->P1, p.a, 128));
+    AFQMC_TRY(maps_for(p1.tf32, p.a, 128));
     AFQMC_TRY(maps_for(m->Sst, p.b, 64, W));
     p.m = M; p.n = N; p.k = M; p.a_batched = 0; p.b_batched = 1;
     p.alpha = cmk(1, 0);
@@ -1727,7 +1745,7 @@ int propagate_mixed(cudaStream_t s, MixedHam* m, const void* P1, bool p1_real, c
   // S = P1 * TMN
   {
     TcParams p{};
-    AFQMC_TRY(maps_for(m->P1, p.a, 128));
+    AFQMC_TRY(maps_for(p1.tf32, p.a, 128));
     AFQMC_TRY(maps_for(m->Tacc_split, p.b, 64, W));
     p.m = M; p.n = N; p.k = M; p.a_batched = 0; p.b_batched = 1;
     p.alpha = cmk(1, 0);

@@ -14,9 +14,14 @@ void mixed_ham_destroy(MixedHam* m);
 int vbias_mixed(cudaStream_t s, MixedHam* m, const c128* G, long ldG, c128* v, int W, double a);
 // split planes of a * X L^T kept in m; V != nullptr also receives them as complex128 [W][M][M]
 int vhs_mixed(cudaStream_t s, MixedHam* m, const c128* X, c128* V, int W, double a);
-// S <- P1 exp_T(iV) P1 S with V from the last vhs_mixed call (P1 real float64 [M][M])
-int propagate_mixed(cudaStream_t s, MixedHam* m, const void* P1, bool p1_real, c128* S, long ldS,
-                    int W, int M, int N, int order);
+// split planes of a one-body propagator (one spin block), kept by the propagator beside its P1
+struct MixedP1;
+void mixed_p1_destroy(MixedP1* p);
+// S <- P1 exp_T(iV) P1 S with V from the last vhs_mixed call (P1 real float64 [M][M]).  *planes is
+// made from P1 on its first use in V's format (null before) and taken as P1's from then on: destroy it
+// with the P1 that it came from.
+int propagate_mixed(cudaStream_t s, MixedHam* m, MixedP1** planes, const void* P1, bool p1_real,
+                    c128* S, long ldS, int W, int M, int N, int order);
 // 0: one batched GEMM launch per Taylor product; 1 (default): all products of a walker in one
 // persistent kernel (M <= 256, N <= 64), one or two walkers in flight per CTA chosen by the walker
 // count; 2 / 3: the persistent kernel with one / two walkers in flight; 4 / 5: the same in the

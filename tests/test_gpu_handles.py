@@ -1,0 +1,89 @@
+"""What the handles keep between calls follows what they were given: several propagators of one
+Hamiltonian, mean fields that change, captured steps beside other calls, host threads."""
+import numpy as np
+import pytest
+import torch
+
+from safire_b200.synth import make_workload
+from tests.gpu_helpers import rand_c, rel_err, to_dev, to_host
+
+pytestmark = pytest.mark.gpu
+# one mixed-precision step against complex128 (operands of 22 bits, FP32 sums); the propagators of two
+# time steps below differ by a percent
+TOL_STEP = 1e-5
+
+
+def _system():
+    """M = 48 (both plane formats), its Hamiltonian handle and some field uniforms."""
+    from safire_b200 import afqmc as A
+    wl = make_workload("cfg1", W=8, M=48, N=6, Nc=40)
+    ham = A.HamiltonianOperations(wl.walker_type, wl.M, wl.nup, wl.ndn, wl.Likn, wl.hij, wl.E0,
+                                  wl.PsiT)
+    u = to_dev(np.random.default_rng(3).random((wl.W, wl.Nc)), torch.float64)
+    return wl, ham, u
+
+
+def _walkers(wl, ham):
+    from safire_b200 import afqmc as A
+    ws = A.WalkerSet(wl.walker_type, wl.M, wl.nup, wl.ndn, wl.W)
+    ws.init_from_trial(ham)
+    A.NOMSD(ham).Energy(ws, set_properties=True)
+    ws.setProperty(A.capi.PSEUDO_ELOC, sum(ws.getProperty(p) for p in
+                                           (A.capi.E1, A.capi.EXX, A.capi.EJ)))
+    return ws
+
+
+def _step(wl, ham, prop, u):
+    ws = _walkers(wl, ham)
+    prop.Propagate(ws, 0.0, u)
+    return to_host(ws.SlaterMatrices(0)).copy()
+
+
+@pytest.mark.parametrize("mode", [0, 2, 4])  # a launch per product, fused TF32, fused FP16
+def test_mixed_step_takes_its_own_propagator(cuda, mode):
+    """Mixed steps of propagators that follow one another on a Hamiltonian (another time step after
+    the first is gone, whose memory the second is likely to get; two at a time, in turn; another
+    mean field) each apply their own exp(-dt H1 / 2), as the complex128 steps do."""
+    from safire_b200 import afqmc as A
+    wl, ham, u = _system()
+    ham.set_taylor_fused(mode)
+
+    def new(dt, precision):
+        return A.Propagator(ham, A.default_params(dt=dt, precision=precision), wl.W)
+
+    want = {dt: _step(wl, ham, new(dt, A.PREC_FP64), u) for dt in (0.01, 0.05)}
+    assert rel_err(want[0.01], want[0.05]) > 100 * TOL_STEP
+    for dt in (0.01, 0.05, 0.01):
+        prop = new(dt, A.PREC_MIXED)
+        assert rel_err(_step(wl, ham, prop, u), want[dt]) < TOL_STEP, dt
+        del prop
+    props = {dt: new(dt, A.PREC_MIXED) for dt in want}
+    for _ in range(2):
+        for dt, prop in props.items():
+            assert rel_err(_step(wl, ham, prop, u), want[dt]) < TOL_STEP, dt
+    # the mean field moves between the one-body propagator and the fields
+    vMF = props[0.05].P1_vMF()[1] + 0.3
+    ref = new(0.05, A.PREC_FP64)
+    ref.set_trial(None, vMF)
+    moved = _step(wl, ham, ref, u)
+    assert rel_err(moved, want[0.05]) > 100 * TOL_STEP
+    props[0.05].set_trial(None, vMF)
+    assert rel_err(_step(wl, ham, props[0.05], u), moved) < TOL_STEP
+    assert ham.device_error_flag() == 0
+
+
+def test_captured_mixed_step_beside_another_propagator(cuda):
+    """A captured mixed step keeps its propagator while another one of the Hamiltonian steps."""
+    from safire_b200 import afqmc as A
+    wl, ham, u = _system()
+    ham.set_taylor_fused(4)
+    a, b = (A.Propagator(ham, A.default_params(dt=dt, precision=A.PREC_MIXED), wl.W)
+            for dt in (0.01, 0.05))
+    want = _step(wl, ham, a, u)
+    ws, eshift = _walkers(wl, ham), torch.zeros(1, dtype=torch.float64, device=cuda)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        a.Propagate_dev(ws, eshift, u)
+    _step(wl, ham, b, u)
+    g.replay()
+    assert np.array_equal(to_host(ws.SlaterMatrices(0)), want)
