@@ -8,7 +8,9 @@
 //   Kl[w,n] = sum_a T[w,a,n,a];   EJ[w] = sclj/2 sum_n Kl[w,n]^2
 // with scl = 2 (CLOSED) or 1, sclj = 4 (CLOSED) or 1.  The reference materialises T in chunks of
 // Cholesky vectors sized by max_memory_MB; the complex128 path here materialises it in chunks of
-// walkers (one DMMA GEMM per chunk) and reduces each N x N block of T with one CTA.
+// walkers (one DMMA GEMM per chunk) and reduces the N x N blocks of T in shared memory.
+#include <algorithm>
+
 #include "energy.cuh"
 #include "mixed.cuh"
 #include "zgemm.cuh"
@@ -62,19 +64,22 @@ __global__ void __launch_bounds__(XB_THREADS)
           acc = cadd(acc, cmul(x, tv[a * pitch + b]));
         }
       }
-  __shared__ double red[4][XB_THREADS / 32];
+  // the warps' sums take the blocks' place, so that N = 120 fits: its block leaves 128 bytes of an SM
+  __syncthreads();
+  double* red = reinterpret_cast<double*>(smem_raw);  // [4][XB_THREADS / 32]
+  constexpr int NW = XB_THREADS / 32;
   double s4[4] = {2 * acc.x + dia.x, 2 * acc.y + dia.y, tr.x, tr.y};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     double x = s4[q];
     for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-    if (lane == 0) red[q][warp] = x;
+    if (lane == 0) red[q * NW + warp] = x;
   }
   __syncthreads();
   if (threadIdx.x < nb) {
     double s[4] = {0, 0, 0, 0};
     for (int q = 0; q < 4; ++q)
-      for (int k = 0; k < GW; ++k) s[q] += red[q][threadIdx.x * GW + k];
+      for (int k = 0; k < GW; ++k) s[q] += red[q * NW + threadIdx.x * GW + k];
     const long o = long(w_first + wl) * Nc + n0 + threadIdx.x;
     exx_part[o] = cadd(exx_part[o], cmk(s[0], s[1]));
     Kl[o] = cadd(Kl[o], cmk(s[2], s[3]));
@@ -84,7 +89,8 @@ __global__ void __launch_bounds__(XB_THREADS)
 template <int NB>
 int launch_exchange_block(cudaStream_t s, const c128* T, int N, int Nc, int w_first, int wc,
                           c128* exx_part, c128* Kl) {
-  const size_t smem = size_t(NB) * N * (N | 1) * sizeof(c128);
+  const size_t sums = 4 * (XB_THREADS / 32) * sizeof(double);
+  const size_t smem = std::max(size_t(NB) * N * (N | 1) * sizeof(c128), sums);
   if (smem > 48 * 1024)
     AFQMC_CUDA_TRY(cudaFuncSetAttribute(exchange_block_kernel<NB>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from tests.gpu_helpers import rand_c, to_dev, to_host
+from tests.gpu_helpers import rand_c, rel_err, to_dev, to_host
 
 pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -53
@@ -254,3 +254,23 @@ def test_mixed_vbias_ranges(cuda, M, N, Nc, W, fmt):
     v, r = to_host(v), to_host(r)
     bound = 8 * (2.0 ** -21 + N * M / 16 * 2.0 ** -23)
     assert np.max(np.abs(v - r)) < bound * np.sqrt(np.mean(np.abs(r) ** 2))
+
+
+@pytest.mark.parametrize("nup,ndn", [(1, 1), (16, 15), (23, 24), (33, 34), (47, 48), (67, 66), (119, 1),
+                                     (120, 120)])
+def test_energy_block_sums(cuda, nup, ndn):
+    """The complex128 energy at the sizes around which a CTA of its block sums takes eight, four, two
+    and one Cholesky vectors, up to the 120 electrons whose block fills an SM's shared memory."""
+    from oracle import afqmc as O
+    from safire_b200 import afqmc as A
+    M, Nc, W = max(nup, ndn) + 1, 11, 3
+    rs = np.random.default_rng(nup)
+    L = rs.standard_normal((M, M, Nc))
+    args = (A.COLLINEAR, M, nup, ndn, (L + L.transpose(1, 0, 2))[None],
+            np.eye(M)[None].astype(complex), 0.0,
+            [np.linalg.qr(rs.standard_normal((M, n)))[0].T.astype(complex) for n in (nup, ndn)])
+    G = rand_c(rs, W, (nup + ndn) * M)
+    E = torch.zeros((W, 3), dtype=torch.complex128, device=cuda)
+    A.HamiltonianOperations(*args).energy(E, to_dev(G))
+    # each of the products' sums has M terms, each energy N^2 Nc of their products
+    assert rel_err(to_host(E), O.Real3IndexFactorization(*args).energy(G)) < 50 * (M + nup) * EPS
