@@ -380,7 +380,11 @@ int afqmc_prop_get_p1(afqmc_prop prop, afqmc_c128* P1, afqmc_c128* vMF);
  * restated as a kernel with the same formula).
  *   uniforms: device [W][Nc] field uniforms (the reference's RNGbuff, rng_block_size = Nc), or
  *             NULL to draw them on the device from the propagator's counter-based generator.
- * Capturable in a CUDA graph when uniforms == NULL or points to a fixed device buffer. */
+ * Capturable in a CUDA graph when uniforms == NULL or points to a fixed device buffer, once a step
+ * of this propagator on these walkers has run (it allocates what later ones use).  The graph holds
+ * the addresses of the handles' buffers: it is good until a handle of the step is destroyed, the
+ * propagator gets another trial or mean field, or a call with more walkers on the step's
+ * Hamiltonian or trial makes the buffers grow (afqmc_phmsd_density_matrix says up to where). */
 int afqmc_prop_step(afqmc_prop prop, afqmc_wset ws, double Eshift, const double* uniforms,
                     afqmc_stream stream);
 /* Same as afqmc_prop_step but Eshift is read from device memory at run time (graph friendly). */
@@ -532,7 +536,8 @@ int afqmc_phmsd_energy(afqmc_phmsd trial, const afqmc_c128* wbuf, long ldS, afqm
  * nact_dn][M] (device, written) = (R_s^T G_s^ref) / Ov per spin block, with R the coefficient-
  * weighted Woodbury matrices of every excited determinant (calculate_R,
  * phmsd_helpers.hpp:200-309); ovlp [W] (device, written) the log overlap.  Blocks of `block`
- * walkers (<= 0: 512). */
+ * walkers (<= 0: at least 512, more as far as their buffers fit 512 MiB).  The handle keeps the
+ * buffers of its largest block; with block <= 0 they are not replaced once they hold 512 walkers. */
 int afqmc_phmsd_density_matrix(afqmc_phmsd trial, const afqmc_c128* wbuf, long ldS,
                                afqmc_c128* G, afqmc_c128* ovlp, int W, int block,
                                afqmc_stream stream);

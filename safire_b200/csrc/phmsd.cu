@@ -2677,24 +2677,28 @@ extern "C" int afqmc_phmsd_density_matrix(afqmc_phmsd h, const afqmc_c128* wbuf,
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   // the density matrix needs only the per-walker Woodbury buffers: blocks of at least 512 walkers,
   // more as far as they fit 512 MiB (0.5 MB a walker at nel = 30, nact = 70, 2000 excitations;
-  // 20 KB at nel = 7, nact = 15, where 1536 walkers in one block take a third of the launches)
+  // 20 KB at nel = 7, nact = 15, where 1536 walkers in one block take a third of the launches).
+  // Buffers of 512 walkers or more are not replaced: larger calls take blocks of what they hold, so
+  // that a captured step of such a population keeps its addresses.
+  constexpr int SETTLED = 512;
   const size_t na = std::max(h->nact[0], h->nact[1]), ne = std::max(h->nel[0], h->nel[1]);
   const size_t per_walker =
       sizeof(c128) * (2 * ne * h->M + 4 * na * ne + ne * ne + h->nuniq[0] + h->nuniq[1] +
                       2 * std::max(h->nuniq[0], h->nuniq[1]) +
                       (3 * size_t(std::max(h->ninv[0], h->ninv[1])) + 1) / 2 + 2);
-  const size_t fit = std::min<size_t>(std::max<size_t>(512, (size_t(512) << 20) / per_walker),
+  const size_t fit = std::min<size_t>(std::max<size_t>(SETTLED, (size_t(512) << 20) / per_walker),
                                       65535);
-  int Wb = block > 0 ? (block < W ? block : W) : int(std::min<size_t>(W, fit));
+  const int most = h->capCore >= SETTLED ? h->capCore : int(fit);
+  int Wb = std::min(W, block > 0 ? block : most);
   // where more than 512 walkers' buffers cannot be had (a capture under way, memory taken): 512
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(s, &cap);
   if (block <= 0 && cap != cudaStreamCaptureStatusNone && h->capCore < Wb)
-    Wb = std::min(Wb, std::max(512, h->capCore));
+    Wb = std::min(Wb, SETTLED);
   int st = phmsd_core_scratch(h, Wb);
-  if (st == AFQMC_ERR_ALLOC && block <= 0 && Wb > 512) {
+  if (st == AFQMC_ERR_ALLOC && block <= 0 && Wb > SETTLED) {
     cudaGetLastError();
-    Wb = 512;
+    Wb = SETTLED;
     st = phmsd_core_scratch(h, Wb);
   }
   if (st) {

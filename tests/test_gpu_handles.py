@@ -87,3 +87,79 @@ def test_captured_mixed_step_beside_another_propagator(cuda):
     _step(wl, ham, b, u)
     g.replay()
     assert np.array_equal(to_host(ws.SlaterMatrices(0)), want)
+
+
+def _phmsd():
+    from safire_b200 import afqmc as A
+    from safire_b200.synth import make_hamiltonian, make_phmsd_trial
+    M, nup, ndn, Nc = 12, 3, 2, 10
+    h1, Likn = make_hamiltonian(M, Nc, 0.9, seed=7)
+    _, C = np.linalg.eigh(h1)
+    t = make_phmsd_trial(M, nup, ndn, C, nocc=2, nvirt=4, ndet=12, seed=3, max_level=2)
+    hij = h1[None].astype(complex)
+    ph = A.PHMSD(t)
+    ph.set_hamiltonian(Likn[None], hij, 0.2)
+    return t, C, hij, Likn, ph
+
+
+def _phmsd_G(ph, C, W, block=0, seed=1):
+    M, n = C.shape[0], (3, 2)
+    rs = np.random.default_rng(seed)
+    S = [C[None, :, :k] + rand_c(rs, W, M, k, scale=0.2 / np.sqrt(M)) for k in n]
+    wbuf = to_dev(np.concatenate([x.reshape(W, -1) for x in S], 1))
+    G = torch.empty((W, sum(ph.info()[3:5]), M), dtype=torch.complex128, device="cuda")
+    ov = torch.empty(W, dtype=torch.complex128, device="cuda")
+    return wbuf, G, ov, lambda: ph.MixedDensityMatrix(wbuf, G, ov, block=block)
+
+
+def test_phmsd_captured_step_beside_larger_calls(cuda):
+    """A captured step of 600 walkers with a particle-hole trial, after the density matrix of 1200 on
+    the same handle: the buffers of 512 and more walkers are not replaced, so its replays write where
+    the capture did, bit for bit what an eager step gives."""
+    from safire_b200 import afqmc as A
+    t, C, hij, Likn, ph = _phmsd()
+    W = 600
+    ham = A.HamiltonianOperations(A.COLLINEAR, t.M, t.nup, t.ndn, Likn[None], hij, 0.2,
+                                  [t.orbmat[s][t.refc[s]] for s in (0, 1)])
+    prop = A.Propagator(ham, A.default_params(dt=0.01), W)
+    prop.set_trial(ph)
+    u = to_dev(np.random.default_rng(4).random((W, ham.Nc)), torch.float64)
+    eshift = torch.zeros(1, dtype=torch.float64, device=cuda)
+
+    def walkers():
+        ws = A.WalkerSet(A.COLLINEAR, t.M, t.nup, t.ndn, W)
+        ws.init_from_trial(ham)
+        return ws
+    eager, ws = walkers(), walkers()
+    prop.Propagate_dev(eager, eshift, u)
+    want = to_host(eager.buffer).copy()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        prop.Propagate_dev(ws, eshift, u)
+    _, G, ov, call = _phmsd_G(ph, C, 2 * W)
+    call()
+    big = to_host(G).copy()
+    g.replay()
+    assert np.array_equal(to_host(ws.buffer), want)
+    call()
+    assert np.array_equal(to_host(G), big)
+
+
+@pytest.mark.parametrize("W", [512, 513, 1300])
+def test_phmsd_density_matrix_captured(cuda, W):
+    """The density matrix under capture: with the buffers of a smaller call it runs in blocks of what
+    they hold, with its own in one, and both give what blocks of 100 give."""
+    _, C, _, _, ph = _phmsd()
+    _, G, _, call = _phmsd_G(ph, C, W, block=100)
+    call()
+    want = to_host(G).copy()
+    for first in (512, W):
+        ph = _phmsd()[-1]
+        _phmsd_G(ph, C, first)[-1]()
+        _, G, _, call = _phmsd_G(ph, C, W)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            call()
+        g.replay()
+        assert np.array_equal(to_host(G), want), first
