@@ -83,6 +83,18 @@ inline int launch_status(const char* what) {
   return AFQMC_OK;
 }
 
+// Room for `bytes` of dynamic shared memory in a launch of kern.  The limit belongs to the kernel on its
+// device, where the calls of several host threads meet, so each of them sets the same one: `most`,
+// the largest that any launch of this kernel asks for.  Without it a block has 48 KB, its static shared
+// memory (below 16 KB in these kernels) included.
+template <class K>
+inline int allow_smem(K* kern, size_t bytes, size_t most) {
+  if (bytes > 32 * 1024)
+    AFQMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        int(bytes > most ? bytes : most)));
+  return AFQMC_OK;
+}
+
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace afqmc

@@ -40,6 +40,7 @@ __device__ __forceinline__ c128 log_pivot(c128 d, bool swapped) {
 // no element read after another thread wrote it in the same phase.
 // ---------------------------------------------------------------------------------------------
 constexpr int GJ_THREADS = 256;
+constexpr size_t GJ_SMEM_MAX = 227 * 1024 - 64;  // an SM's shared memory less the statics
 
 template <bool INVERT>
 __global__ void __launch_bounds__(GJ_THREADS) gj_logdet_kernel(const c128* __restrict__ A,
@@ -764,13 +765,11 @@ int batched_logdet_inverse(cudaStream_t s, const c128* A, long strideA, c128* Ai
     }
     const size_t smem = gb_smem(N);
     if (invert) {
-      AFQMC_CUDA_TRY(cudaFuncSetAttribute(gj_block_kernel<true>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      AFQMC_TRY(allow_smem(gj_block_kernel<true>, smem, gb_smem(64)));
       gj_block_kernel<true><<<W, GB_THREADS, smem, s>>>(A, strideA, Ainv, strideInv, ovlp, N,
                                                         post_scale, post_add);
     } else {
-      AFQMC_CUDA_TRY(cudaFuncSetAttribute(gj_block_kernel<false>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      AFQMC_TRY(allow_smem(gj_block_kernel<false>, smem, gb_smem(64)));
       gj_block_kernel<false><<<W, GB_THREADS, smem, s>>>(A, strideA, nullptr, 0, ovlp, N,
                                                          post_scale, post_add);
     }
@@ -784,13 +783,11 @@ int batched_logdet_inverse(cudaStream_t s, const c128* A, long strideA, c128* Ai
     return AFQMC_ERR_UNSUPPORTED;
   }
   if (invert) {
-    AFQMC_CUDA_TRY(cudaFuncSetAttribute(gj_logdet_kernel<true>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    AFQMC_TRY(allow_smem(gj_logdet_kernel<true>, smem, GJ_SMEM_MAX));
     gj_logdet_kernel<true><<<W, GJ_THREADS, smem, s>>>(A, strideA, Ainv, strideInv, ovlp, N,
                                                        post_scale, post_add);
   } else {
-    AFQMC_CUDA_TRY(cudaFuncSetAttribute(gj_logdet_kernel<false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    AFQMC_TRY(allow_smem(gj_logdet_kernel<false>, smem, GJ_SMEM_MAX));
     gj_logdet_kernel<false><<<W, GJ_THREADS, smem, s>>>(A, strideA, nullptr, 0, ovlp, N,
                                                         post_scale, post_add);
   }

@@ -91,9 +91,7 @@ int launch_exchange_block(cudaStream_t s, const c128* T, int N, int Nc, int w_fi
                           c128* exx_part, c128* Kl) {
   const size_t sums = 4 * (XB_THREADS / 32) * sizeof(double);
   const size_t smem = std::max(size_t(NB) * N * (N | 1) * sizeof(c128), sums);
-  if (smem > 48 * 1024)
-    AFQMC_CUDA_TRY(cudaFuncSetAttribute(exchange_block_kernel<NB>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  AFQMC_TRY(allow_smem(exchange_block_kernel<NB>, smem, NB == 1 ? 227 * 1024 : XB_SMEM));
   exchange_block_kernel<NB><<<dim3(ceil_div(Nc, NB), wc), XB_THREADS, smem, s>>>(T, N, Nc, w_first,
                                                                                 exx_part, Kl);
   return launch_status("exchange_block_kernel");

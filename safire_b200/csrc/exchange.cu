@@ -355,8 +355,7 @@ int make_plane_map_3d_es(CUtensorMap* map, const void* base, int esize, long k, 
 namespace {
 template <int SA, int NSPLIT, bool F16>
 int launch_exchange(cudaStream_t s, const XParams& p, int grid, size_t smem) {
-  AFQMC_CUDA_TRY(cudaFuncSetAttribute(exchange_tc_kernel<SA, NSPLIT, F16>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  AFQMC_TRY(allow_smem(exchange_tc_kernel<SA, NSPLIT, F16>, smem, X_SMEM_MAX));
   exchange_tc_kernel<SA, NSPLIT, F16><<<grid, XT_THREADS, smem, s>>>(p);
   return launch_status("exchange_tc_kernel");
 }

@@ -815,6 +815,7 @@ __global__ void __launch_bounds__(SPLIT_ROW_THREADS) split_walkers_T_f16_kernel(
 // (the second from L2: the walkers in flight are 47 MB at M = 200, N = 50) and whole lines of the planes'
 // rows, where a thread per row i above reads 16 bytes of a line at a time.
 constexpr int SPLIT_T_THREADS = 1024;
+constexpr size_t SPLIT_T_SMEM_MAX = 110 * 1024;
 inline int split_T_pitch(int M) {  // halves: an odd number of words
   const int w = (M + 1) / 2;
   return 2 * (w | 1);
@@ -1659,9 +1660,8 @@ int propagate_mixed(cudaStream_t s, MixedHam* m, MixedP1** planes, const void* P
       p1.f16 = f16;
     }
     const size_t tsm = split_T_smem(M, N);
-    if (tsm <= 110 * 1024) {
-      AFQMC_CUDA_TRY(cudaFuncSetAttribute(split_walkers_T_f16_tile_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(tsm)));
+    if (tsm <= SPLIT_T_SMEM_MAX) {
+      AFQMC_TRY(allow_smem(split_walkers_T_f16_tile_kernel, tsm, SPLIT_T_SMEM_MAX));
       split_walkers_T_f16_tile_kernel<<<W, SPLIT_T_THREADS, tsm, s>>>(
           S, ldS, M, N, m->Sst16.h(0), m->Sst16.h(1), m->Sst16.h(2), m->Sst16.h(3), m->Sst16.ld,
           m->Sst16.bstride(), m->s_inv, split_T_pitch(M));

@@ -28,6 +28,7 @@ namespace {
 
 constexpr int PH_THREADS = 256;
 constexpr int PH_NEX_MAX = 8;
+constexpr size_t PH_SMEM_MAX = 200 * 1024;  // a CTA's dynamic shared memory (but for the groups kernel)
 
 // complex arithmetic in single precision for the mixed-precision energy tables (the complex128
 // helpers of common.cuh, restated for float2)
@@ -1050,6 +1051,7 @@ __global__ void __launch_bounds__(PHX_THREADS, sizeof(R) == 4 ? 2 : 1) excited_e
 // no faster.
 constexpr int PHG_THREADS = 384;
 constexpr int PHG_N = 8;
+constexpr size_t PHG_SMEM_MAX = 225 * 1024;
 constexpr int PHG_RT = 4, PHG_CT = 4;  // rows and columns of a thread's product tile
 
 using f2 = unsigned long long;  // two packed floats
@@ -1697,12 +1699,11 @@ extern "C" int afqmc_ph_excited_2body_energy(const int* iexcit, const int* refc,
   AFQMC_TRY(check_indices("afqmc_ph_excited_2body_energy", reinterpret_cast<cudaStream_t>(stream),
                           iexcit, refc, ndet, nex, nact, nelec));
   const size_t smem = size_t(nex) * nact * sizeof(c128) + 2 * size_t(nelec) * sizeof(int);
-  if (smem > 200 * 1024) {
+  if (smem > PH_SMEM_MAX) {
     set_error_detail("afqmc_ph_excited_2body_energy: nex*nact too large (%d x %d)", nex, nact);
     return AFQMC_ERR_UNSUPPORTED;
   }
-  AFQMC_CUDA_TRY(cudaFuncSetAttribute(ph_excited_2body_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  AFQMC_TRY(allow_smem(ph_excited_2body_kernel, smem, PH_SMEM_MAX));
   dim3 grid(ndet, nw);
   ph_excited_2body_kernel<<<grid, PH_THREADS, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
       iexcit, refc, reinterpret_cast<const c128*>(Twina), reinterpret_cast<const c128*>(R),
@@ -2388,7 +2389,7 @@ size_t excited_tables_smem(afqmc_phmsd h, int sp, size_t elem, int ng, int nbuf)
 // the energy of spin sp runs the per-(walker, n) tables kernel (else the per-shell R rows)
 bool phmsd_tables(afqmc_phmsd h, int sp) {
   const size_t esz = h->precision == AFQMC_PREC_MIXED ? sizeof(c64) : sizeof(c128);
-  return h->tables_ok[sp] && excited_tables_smem(h, sp, esz, 1, 1) <= 200 * 1024;
+  return h->tables_ok[sp] && excited_tables_smem(h, sp, esz, 1, 1) <= PH_SMEM_MAX;
 }
 
 // the FP16 split planes of Lnak for the mixed half rotation, made at the first mixed energy
@@ -2466,8 +2467,7 @@ int phmsd_reference_and_excited(afqmc_phmsd h, cudaStream_t s, int sp, int nb, d
     AFQMC_TRY(launch_status("ph_excited_1body_kernel"));
     c128* KE = cross ? h->KEl : KEout + size_t(k0) * nb * Nc;
     const size_t smem = size_t(nex) * na * sizeof(c128) + 2 * size_t(N) * sizeof(int);
-    AFQMC_CUDA_TRY(cudaFuncSetAttribute(ph_excited_2body_kernel,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    AFQMC_TRY(allow_smem(ph_excited_2body_kernel, smem, PH_SMEM_MAX));
     ph_excited_2body_kernel<<<grid, PH_THREADS, smem, s>>>(iex, h->refc[sp], h->Twina, h->R, w,
                                                           nb, nd, nex, na, N, Nc, h->el + nb,
                                                           h->el + 2 * nb, KE);
@@ -2487,8 +2487,7 @@ int phmsd_reference_and_excited(afqmc_phmsd h, cudaStream_t s, int sp, int nb, d
           h->uhdrs[sp]);
       AFQMC_TRY(launch_status("woodbury_inverses_kernel"));
       const size_t sm1 = size_t(N) * h->nv[sp] * sizeof(c128);
-      AFQMC_CUDA_TRY(cudaFuncSetAttribute(excited_1body_all_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm1)));
+      AFQMC_TRY(allow_smem(excited_1body_all_kernel, sm1, PH_SMEM_MAX));
       excited_1body_all_kernel<<<dim3(nb, 4), PH_THREADS, sm1, s>>>(
           h->Swia, h->eQ[sp], h->refc[sp], h->vl[sp], h->nv[sp], h->uhdr[sp], h->uexc4[sp],
           h->INV, h->ninv[sp], h->wgt, h->nuniq[sp], nb, N, na, h->el);
@@ -2505,7 +2504,7 @@ int phmsd_reference_and_excited(afqmc_phmsd h, cudaStream_t s, int sp, int nb, d
     // weight are then read once per four indices), the next index's rows loaded while the
     // current tables are built where a second row buffer fits
     const size_t esz = mixed ? sizeof(c64) : sizeof(c128);
-    const size_t lim = size_t(mixed ? 110 : 200) * 1024;
+    const size_t lim = mixed ? 110 * 1024 : PH_SMEM_MAX;
     int ngr = 4, nbuf = 2;
     if (excited_tables_smem(h, sp, esz, 4, 2) > lim) nbuf = 1;
     if (excited_tables_smem(h, sp, esz, 4, nbuf) > lim) ngr = nbuf = 1;
@@ -2514,8 +2513,7 @@ int phmsd_reference_and_excited(afqmc_phmsd h, cudaStream_t s, int sp, int nb, d
     // the K vectors have Twina's element type (complex64 in the mixed energy's tables path)
     auto go = [&](auto kern, const auto* tw, const auto* inv) -> int {
       using KT = std::remove_const_t<std::remove_pointer_t<decltype(tw)>>;
-      AFQMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(smem)));
+      AFQMC_TRY(allow_smem(kern, smem, PH_SMEM_MAX));
       kern<<<grid, PHX_THREADS, smem, s>>>(
           tw, h->eQ[sp], h->refc[sp], h->hl[sp], h->vl[sp], h->nh[sp], h->nv[sp],
           mixed ? h->uhdrs[sp] : h->uhdr[sp], mixed ? h->uexc4s[sp] : h->uexc4[sp], inv,
@@ -2539,9 +2537,8 @@ int phmsd_reference_and_excited(afqmc_phmsd h, cudaStream_t s, int sp, int nb, d
     };
     const c128* twd = h->Twina;
     const size_t gsm = excited_groups_smem(N, h->nh[sp], h->nv[sp]);
-    if (mixed && h->twina64[sp] && !rare && h->nh[sp] > 0 && gsm <= 225 * 1024) {
-      AFQMC_CUDA_TRY(cudaFuncSetAttribute(excited_energy_groups_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(gsm)));
+    if (mixed && h->twina64[sp] && !rare && h->nh[sp] > 0 && gsm <= PHG_SMEM_MAX) {
+      AFQMC_TRY(allow_smem(excited_energy_groups_kernel, gsm, PHG_SMEM_MAX));
       excited_energy_groups_kernel<<<dim3((Nc + PHG_N - 1) / PHG_N, nb), PHG_THREADS, gsm, s>>>(
           tw64, h->eQ[sp], h->refc[sp], h->hl[sp], h->vl[sp], h->nh[sp], h->nv[sp], h->uhdrs[sp],
           h->uexc4s[sp], inv32, h->ninv[sp], h->wgtT, h->nuniq[sp], nb, N, na, Nc, h->el + nb,
@@ -2742,11 +2739,10 @@ extern "C" int afqmc_phmsd_density_matrix(afqmc_phmsd h, const afqmc_c128* wbuf,
           AFQMC_TRY(launch_status("woodbury_inverses_kernel"));
         }
         const size_t rsm = 3 * size_t(N) * na * sizeof(c128);
-        AFQMC_CHECK_ARG(rsm <= 200 * 1024,
+        AFQMC_CHECK_ARG(rsm <= PH_SMEM_MAX,
                         "afqmc_phmsd_density_matrix: nel x nact = %d x %d exceeds shared memory",
                         N, na);
-        AFQMC_CUDA_TRY(cudaFuncSetAttribute(phmsd_R_kernel,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, int(rsm)));
+        AFQMC_TRY(allow_smem(phmsd_R_kernel, rsm, PH_SMEM_MAX));
         phmsd_R_kernel<<<nb, PHR_THREADS, rsm, s>>>(h->eQ[sp], h->refc[sp], h->hrow[sp],
                                                     h->hent[sp], h->uexc[sp], h->INV,
                                                     h->ninv[sp], h->wgt, nu, nb, N, na, h->Rfull);

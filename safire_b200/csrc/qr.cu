@@ -33,6 +33,8 @@ namespace {
 // ---------------------------------------------------------------------------------------------
 constexpr int CH_THREADS = 128;
 
+constexpr int CH_MAX_N = 85;  // the largest N that orthogonalize takes (shared memory holds 112)
+
 __host__ __device__ inline int ch_pad(int N) { return (N + 7) / 8 * 8; }
 inline size_t ch_smem(int N) { return size_t(ch_pad(N)) * (ch_pad(N) + 1) * sizeof(c128); }
 
@@ -148,8 +150,7 @@ static int cholqr_pass(cudaStream_t s, const c128* S, long ldS, c128* Q, long ld
   g.alpha = cmk(1, 0); g.beta = cmk(0, 0);
   AFQMC_TRY(zgemm(s, W, GH, false, GN, false, g));
   const size_t smem = ch_smem(N);
-  AFQMC_CUDA_TRY(cudaFuncSetAttribute(chol_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(smem)));
+  AFQMC_TRY(allow_smem(chol_inv_kernel, smem, ch_smem(CH_MAX_N)));
   chol_inv_kernel<<<W, CH_THREADS, smem, s>>>(gram, rinv, logdetR, N);
   AFQMC_TRY(launch_status("chol_inv_kernel"));
   GemmParams q{};
@@ -171,8 +172,8 @@ int orthogonalize(cudaStream_t s, c128* S, long ldS, c128* logdetR, int W, int M
     set_error_detail("orthogonalize: N = %d > M = %d", N, M);
     return AFQMC_ERR_SHAPE;
   }
-  if (2 * size_t(N | 1) * N * sizeof(c128) > 227 * 1024) {
-    set_error_detail("orthogonalize: N = %d exceeds the shared-memory Cholesky kernel", N);
+  if (N > CH_MAX_N) {
+    set_error_detail("orthogonalize: N = %d > %d", N, CH_MAX_N);
     return AFQMC_ERR_UNSUPPORTED;
   }
   const size_t nQ = size_t(W) * M * N, nG = size_t(W) * N * N;

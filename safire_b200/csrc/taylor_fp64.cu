@@ -218,9 +218,7 @@ int run(cudaStream_t s, const void* P1, bool p1_real, const c128* V, long stride
   const size_t smem = smem_bytes(M, TN);
   const int threads = 32 * ceil_div(M, 8 * SPW);
   auto go = [&](auto kern) -> int {
-    if (smem > 48 * 1024)
-      AFQMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(smem)));
+    AFQMC_TRY(allow_smem(kern, smem, smem_bytes(SPW == 2 ? 128 : KV > 0 ? 32 : 64, TN)));
     kern<<<W, threads, smem, s>>>(P1, V, strideV, S, ldS, M, N, order);
     return launch_status("taylor_c128_kernel");
   };

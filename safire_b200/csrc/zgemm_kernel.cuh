@@ -283,12 +283,13 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 2) zgemm_kernel(GemmParams p, 
 template <int TN, class O, bool SYM>
 int launch(cudaStream_t s, int batch, const GemmParams& p, const Shape& sh) {
   auto kern = zgemm_kernel<TN, O, SYM>;
-  const int bm = 8 * sh.warps, bn = 8 * TN;
+  constexpr int bn = 8 * TN;
+  const int bm = 8 * sh.warps;
   size_t smem = size_t(STAGES) * O::stage_bytes(bm, bn);
   if (sh.split > 1 && smem < size_t(bm) * bn * sizeof(c128)) smem = size_t(bm) * bn * sizeof(c128);
-  if (smem > 48 * 1024)
-    AFQMC_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        int(smem)));
+  constexpr size_t ring = STAGES * size_t(O::stage_bytes(8 * MAX_WARPS, bn));
+  constexpr size_t sums = size_t(8 * MAX_WARPS) * bn * sizeof(c128);
+  AFQMC_TRY(allow_smem(kern, smem, ring > sums ? ring : sums));  // of any shape
   unsigned gx = ceil_div(p.n, bn);
   if (SYM) {
     const unsigned nb = ceil_div(p.sym_m, 8);

@@ -163,3 +163,87 @@ def test_phmsd_density_matrix_captured(cuda, W):
             call()
         g.replay()
         assert np.array_equal(to_host(G), want), first
+
+
+def _energy_call(M, N, precision):
+    from safire_b200 import afqmc as A
+    rs = np.random.default_rng(N)
+    L = rs.standard_normal((M, M, 24))
+    psi = np.linalg.qr(rs.standard_normal((M, N)))[0].T.astype(complex)
+    ham = A.HamiltonianOperations(A.CLOSED, M, N, N, (L + L.transpose(1, 0, 2))[None],
+                                  np.eye(M)[None].astype(complex), 0.0, [psi])
+    G = to_dev(rand_c(rs, 4, N * M))
+
+    def call():
+        E = torch.zeros((4, 3), dtype=torch.complex128, device="cuda")
+        ham.energy(E, G, precision=precision)
+        return E
+    return call
+
+
+def _det_op_call(name, W, M, N):
+    from safire_b200 import afqmc as A
+    rs = np.random.default_rng(N)
+    S = to_dev(np.eye(M, N) + rand_c(rs, W, M, N, scale=0.3 / np.sqrt(M)))
+    if name == "inverse":
+        A_ = S[:, :N].contiguous()
+
+        def call():
+            inv, ld = torch.empty_like(A_), torch.zeros(W, dtype=torch.complex128, device="cuda")
+            A.det_ops.inverse_logdet(A_, inv, ld)
+            return inv
+    elif name == "orthogonalize":
+        def call():
+            q, ld = S.clone(), torch.zeros(W, dtype=torch.complex128, device="cuda")
+            A.det_ops.orthogonalize(q, ld)
+            return q
+    else:
+        P1 = to_dev(np.eye(M) + rand_c(rs, M, M, scale=0.1 / np.sqrt(M)))
+        V = to_dev(rand_c(rs, W, M, M, scale=0.5 / np.sqrt(M)))
+
+        def call():
+            q = S.clone()
+            A.det_ops.Propagate(q, P1, V)
+            return q
+    return call
+
+
+@pytest.mark.parametrize("kind", ["propagate_gemm", "propagate_fused", "inverse", "orthogonalize",
+                                  "energy", "energy_mixed"])
+def test_host_threads(cuda, kind):
+    """Two host threads, each on a stream of its own, whose calls take the same kernels at sizes that
+    need different amounts of shared memory: every call succeeds and returns what it returns alone."""
+    import threading
+    from safire_b200 import afqmc as A
+    calls = {"propagate_gemm": lambda: [_det_op_call("propagate", 150, 64, 64),
+                                        _det_op_call("propagate", 24, 200, 64)],
+             "propagate_fused": lambda: [_det_op_call("propagate", 4, 128, 32),
+                                         _det_op_call("propagate", 4, 65, 32)],
+             "inverse": lambda: [_det_op_call("inverse", 4, 70, 64), _det_op_call("inverse", 4, 70, 57)],
+             "orthogonalize": lambda: [_det_op_call("orthogonalize", 4, 90, 85),
+                                       _det_op_call("orthogonalize", 4, 70, 64)],
+             "energy": lambda: [_energy_call(104, 100, A.PREC_FP64), _energy_call(104, 60, A.PREC_FP64)],
+             "energy_mixed": lambda: [_energy_call(104, 50, A.PREC_MIXED),
+                                      _energy_call(104, 33, A.PREC_MIXED)]}[kind]()
+    want = [c() for c in calls]
+    torch.cuda.synchronize()
+    errors, start = [], threading.Barrier(len(calls))
+
+    def run(call, expect):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait()
+                for _ in range(150):
+                    got = call()
+                torch.cuda.current_stream().synchronize()
+                if not torch.equal(got, expect):
+                    errors.append(f"another result: {(got - expect).abs().max().item():.2e}")
+        except Exception as e:  # raised again on the test's own thread
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=run, args=a) for a in zip(calls, want)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
