@@ -95,6 +95,8 @@ inline int allow_smem(K* kern, size_t bytes, size_t most) {
   return AFQMC_OK;
 }
 
+constexpr int NUM_SMS = 148;  // of a B200: the measure of what fills the device
+
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace afqmc

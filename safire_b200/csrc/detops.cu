@@ -302,7 +302,7 @@ template <int G, int NC>
 void launch_gj_warp(cudaStream_t s, const c128* A, long strideA, c128* Ainv, long strideInv,
                     c128* ovlp, int W, int N, bool invert, c128 post_scale, c128 post_add) {
   // single-warp blocks until every SM has a block's worth, so that few matrices spread out
-  const int nw = ceil_div(W, 32 / G) < 148 * GW_WARPS ? 1 : GW_WARPS;
+  const int nw = ceil_div(W, 32 / G) < NUM_SMS * GW_WARPS ? 1 : GW_WARPS;
   const int grid = ceil_div(W, nw * (32 / G));
   if (invert)
     gj_warp_kernel<G, NC, true><<<grid, 32 * nw, 0, s>>>(A, strideA, Ainv, strideInv, ovlp, W,

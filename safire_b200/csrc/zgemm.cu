@@ -2,6 +2,8 @@
 // zgemm_kernel.cuh, its instantiations in zgemm_*.cu).
 #include "zgemm.cuh"
 
+#include <algorithm>
+
 namespace afqmc {
 namespace zg {
 
@@ -21,8 +23,6 @@ int launch_rtn(cudaStream_t, int, const GemmParams&, const Shape&);
 int launch_nrt_sym(cudaStream_t, const GemmParams&, const Shape&);
 
 namespace {
-
-constexpr int SMS = 148;
 
 // Columns of a tile in units of 8, at most 8 of them: the number that pads n least, where a
 // narrower tile has to save 1/32 of the work per unit given up (it reads A that much more often).
@@ -56,21 +56,64 @@ int fit_rows(int m) {
   return 8;
 }
 
+// Time (cycles) of a single problem in a shape, up to what all shapes share.  A K tile of a CTA costs its
+// SM the DMMAs of the busiest scheduler and the fragment loads of all its warps (x), and takes no less
+// than the latency of a stage, which grows with the copies a thread issues for it; resident CTAs
+// overlap that latency, and what does not fit a wave adds another.  Clusters of four and eight leave
+// about a twelfth of the SMs unused.  The constants are fitted to 2200 timings of 42 problems
+// (1..1536 rows, 60..40000 columns, K = 57..4290).
+double model_time(const Shape& sh, int m, int n, int k, bool a_real, bool b_real) {
+  const int w = sh.warps, tn = sh.tn, c = sh.split;
+  const int frag_a = a_real ? 2 : 4, frag_b = b_real ? 2 : 4;  // wavefronts of a fragment load
+  const int mma = a_real && b_real ? 1 : (a_real || b_real ? 2 : 4);
+  const double x = 0.6 * ((w + 3) / 4 * tn * 4 * mma * 16) + 2.2 * (w * 4 * (frag_a + tn * frag_b));
+  const double latency = 77.0 * (4 + (4 * tn + w - 1) / w) + 0.9 * x;
+  const int ring = STAGES * 8 * (BK + 4) * (w * (a_real ? 8 : 16) + tn * (b_real ? 8 : 16));
+  const int smem = (c > 1 ? std::max(ring, 64 * w * tn * 16) : ring) + 1024;
+  const int resident = std::max(1, std::min(227 * 1024 / smem, 16 / w));
+  const int tiles = (m + 8 * w - 1) / (8 * w) * ((n + 8 * tn - 1) / (8 * tn));
+  const int sms = c > 2 ? NUM_SMS * 11 / 12 : NUM_SMS, per_sm = (tiles * c + sms - 1) / sms;
+  const int waves = per_sm / resident, rest = per_sm - waves * resident;
+  const double cycles = waves * std::max(resident * x, latency) +
+                        (rest ? std::max(rest * x, latency) : 0.0);
+  return cycles * (((k + BK - 1) / BK + c - 1) / c) + (c > 1 ? 3000.0 : 0.0);
+}
+
+// 64 x 64 tiles fill the SMs twice over
+bool many_tiles(int m, long n) { return ceil_div(m, 64) * long(ceil_div(n, 64)) >= 2 * NUM_SMS; }
+
+// The shape for a single problem of few tiles: that of least time by the model, if it saves a tenth of
+// the fitted tiles' time.  K is split in two K tiles or more each, and not where there are many tiles.
+// On the problems above the choice is within 8.6% of the fastest shape in the mean, 35% at worst.  The
+// fitted tiles, with K split in eight K tiles or more, took 1.5 times as long: 1024 x 400 x 4160
+// (real B) in tiles of 64 x 40 is 160 CTAs, two on 12 of the SMs and one on the others (462 us, now
+// 335), and 1 x 4096 x 200 one warp an SM (27.5 us, now 11).
+Shape least_time(Shape fit, int m, int n, int k, bool a_real, bool b_real) {
+  const int ktiles = ceil_div(k, BK);
+  const bool may_split = !many_tiles(m, n);
+  double least = 0.9 * model_time(fit, m, n, k, a_real, b_real);
+  for (int w = m >= 64 ? 4 : 1; w <= 8 && (w <= 2 || m > 4 * w); w *= 2)
+    for (int tn = 1; tn <= 8 && n > 8 * (tn - 1); ++tn)
+      for (int c = 1; c <= 8 && (c == 1 || (may_split && ktiles >= 2 * c)); c *= 2) {
+        const double t = model_time({w, tn, c}, m, n, k, a_real, b_real);
+        if (t < least) {
+          least = t;
+          fit = {w, tn, c};
+        }
+      }
+  return fit;
+}
+
 }  // namespace
 
-// The CTA shape: tiles fitted to m and n; then, where those are too few to give every SM one, the
-// K range of a single problem split over a cluster of up to 8 CTAs (each keeping at least 8 K
-// tiles, so that the reduction stays small against the product), and the tiles halved down to 8
-// strips in all (below that the operand loads bound a tile).
-Shape shape(int batch, int m, int n, int k) {
+// The CTA shape: tiles fitted to m and n; where those of a batch are too few to give every SM one,
+// halved down to 8 strips in all (below that the operand loads bound a tile).  A single problem of few
+// tiles takes the shape of least time.
+Shape shape(int batch, int m, int n, int k, bool a_real, bool b_real) {
   Shape sh{fit_rows(m), fit_cols(n), 1};
   auto ctas = [&] { return long(ceil_div(m, 8 * sh.warps)) * ceil_div(n, 8 * sh.tn) * batch; };
-  if (batch == 1 && ctas() < SMS) {
-    const long s = SMS / ctas(), ks = ceil_div(k, 16) / 8;
-    const long c = s < ks ? s : ks;
-    sh.split = int(c < 1 ? 1 : (c > 8 ? 8 : c));
-  }
-  while (ctas() * sh.split < SMS && sh.warps * sh.tn > 8) {
+  if (batch == 1 && ctas() < 5 * NUM_SMS) return least_time(sh, m, n, k, a_real, b_real);
+  while (ctas() < NUM_SMS && sh.warps * sh.tn > 8) {
     if (sh.tn >= sh.warps)
       sh.tn = (sh.tn + 1) / 2;
     else
@@ -122,7 +165,7 @@ int zgemm(cudaStream_t s, int batch, GemmTrans ta, bool a_real, GemmTrans tb, bo
         int(a_real), int(tb), int(b_real));
     return AFQMC_ERR_UNSUPPORTED;
   }
-  return fn(s, batch, p, zg::shape(batch, p.m, p.n, p.k));
+  return fn(s, batch, p, zg::shape(batch, p.m, p.n, p.k, a_real, b_real));
 }
 
 int zgemm_sym_pairs(cudaStream_t s, int M, const GemmParams& p) {
@@ -130,11 +173,13 @@ int zgemm_sym_pairs(cudaStream_t s, int M, const GemmParams& p) {
   GemmParams q = p;
   q.sym_m = M;
   q.n = M * M;
-  // Worth it once the blocks fill the SMs twice over: below that the time is one tile's, and the
-  // general form's tiles can be narrower than the 64 pairs of a block.  (1024 walkers, M = 200,
-  // 1600 vectors: 4.73 ms, against 8.6 ms for all pairs.)
+  // Worth it where the general form has many tiles (and does not split its sums): with fewer the time
+  // is one tile's, and the general form's can be narrower than the 64 pairs of a block.  Rows for
+  // fewer than four warps leave a block to the latency of its loads, so two blocks an SM then.
+  // (1024 walkers, M = 200, 1600 vectors: 4.73 ms, against 8.6 ms for all pairs.)
   const long nb = ceil_div(M, 8), blocks = nb * (nb + 1) / 2;
-  if (ceil_div(p.m, 64) * blocks < 2 * zg::SMS) return zgemm(s, 1, GN, false, GT, true, q);
+  if (!zg::many_tiles(p.m, long(M) * M) || (p.m <= 24 && blocks < 2 * NUM_SMS))
+    return zgemm(s, 1, GN, false, GT, true, q);
   zg::Shape sh{zg::fit_rows(p.m), 8, 1};
   if (p.m > 65535l * 8 * sh.warps) sh.warps = 8;
   return zg::launch_nrt_sym(s, q, sh);

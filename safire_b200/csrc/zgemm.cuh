@@ -40,6 +40,8 @@ int zgemm(cudaStream_t stream, int batch, GemmTrans ta, bool a_real, GemmTrans t
 int zgemm_sym_pairs(cudaStream_t stream, int M, const GemmParams& p);
 
 namespace zg {
+constexpr int BK = 16;     // the kernel's K tile
+constexpr int STAGES = 3;  // ... and how many of them a CTA's ring holds
 // CTA shape of a launch: warps (8 output rows each), tn (8 output columns each), K split
 struct Shape {
   int warps, tn, split;

@@ -6,7 +6,7 @@
 // 4 cycles whatever the tile, and one A and TN B fragment loads feed TN (real x real) to 4 TN
 // (complex x complex) of them, so the FP64 rate bounds every shape that fills its tiles.  What is
 // lost is lost to padding: the tile is therefore fitted to the problem in steps of 8 in both
-// directions (zgemm_shape in zgemm.cu) instead of being 64 x 64.
+// directions (shape in zgemm.cu) instead of being 64 x 64.
 //
 // K runs in tiles of 16 through a ring of three shared-memory stages, one barrier per tile; the
 // row pitches are padded so that the fragment loads are free of bank conflicts for 16-byte
@@ -28,8 +28,6 @@
 namespace afqmc {
 namespace zg {
 
-constexpr int BK = 16;
-constexpr int STAGES = 3;
 constexpr int MAX_WARPS = 8;
 
 // one element from global to shared memory, zero when `in` is false (the address is not read)

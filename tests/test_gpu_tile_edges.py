@@ -118,6 +118,28 @@ def test_vhs_vbias_shapes(cuda, W, M, Nc):
     assert np.max(np.abs(to_host(v) - want)) < 20 * N * M * EPS * scale
 
 
+@pytest.mark.parametrize("M,N", [(257, 1), (41, 20), (67, 25), (130, 33)])  # K = N M, 1 to 12 mod 16
+@pytest.mark.parametrize("W", [1, 20, 70, 300])
+@pytest.mark.parametrize("real", [True, False])
+def test_vbias_split_sum(cuda, M, N, W, real):
+    """The force bias where its sum over K is split over CTAs (few walkers and vectors), with a ragged
+    last K tile and numbers of K tiles that the parts do not divide, for real and complex trials."""
+    from safire_b200 import afqmc as A
+    Nc = 37
+    rs = np.random.default_rng(W + M)
+    L = rs.standard_normal((M, M, Nc))
+    psi = np.linalg.qr(rand_c(rs, M, N))[0].T
+    ham = A.HamiltonianOperations(A.CLOSED, M, N, N, (L + L.transpose(1, 0, 2))[None],
+                                  np.eye(M)[None].astype(complex), 0.0,
+                                  [psi.real.astype(complex) if real else psi])
+    G = rand_c(rs, W, N * M)
+    v = torch.zeros((W, Nc), dtype=torch.complex128, device=cuda)
+    ham.vbias(to_dev(G), v, 0.01)
+    Lnak = ham.tensors().Lnak[0].reshape(Nc, N * M)
+    scale = 0.2 * np.max(np.abs(G)) * np.max(np.abs(Lnak))
+    assert np.max(np.abs(to_host(v) - 0.2 * G @ Lnak.T)) < 20 * N * M * EPS * scale
+
+
 @pytest.mark.parametrize("M,N,W,ndet", [(9, 1, 3, 1), (17, 5, 40, 3), (64, 16, 9, 1), (75, 33, 30, 2),
                                        (41, 20, 300, 2)])
 def test_real_trial(cuda, M, N, W, ndet):
