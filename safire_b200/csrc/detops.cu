@@ -172,11 +172,12 @@ __global__ void __launch_bounds__(GJ_THREADS) gj_logdet_kernel(const c128* __res
 // Warp-resident Gauss-Jordan / LU for N <= 16: G lanes (the power of two >= N) hold one matrix, a
 // row per lane and its columns in registers, 32 / G matrices to a warp, no block barriers.
 // Partial pivoting as izamax; the pivots give the log determinant, the in-place Gauss-Jordan the
-// inverse.  Row interchanges move no data: each lane knows the logical index of its row.  The columns are kept rotated so that the pivot column of every step is register 0
-// (the update of column j writes register j - 1, and the finished column goes to register
-// NC - 1), so the step loop is not unrolled over k and no register index depends on N; the NC - N
-// registers past the matrix rotate along as zeros that nothing reads.  The pivot row reaches the
-// other lanes by shuffles (G <= 8) or through a shared-memory row.
+// inverse.  Row interchanges move no data: each lane knows the logical index of its row.  The
+// columns are kept rotated so that the pivot column of every step is register 0 (the update of column
+// j writes register j - 1, and the finished column goes to register NC - 1), so the step loop is not
+// unrolled over k and no register index depends on N; the NC - N registers past the matrix rotate
+// along as zeros that nothing reads.  The pivot row reaches the other lanes by shuffles (G <= 8) or
+// through a shared-memory row.
 // What bounds it is the latency of the N dependent steps; small matrices are many (a trial of 34
 // determinants inverts 52224 of 3 x 3 per spin and step), so the point is matrices in flight: a
 // 128-thread CTA per matrix took 232 us for those, this form 10.4.
@@ -313,11 +314,11 @@ void launch_gj_warp(cudaStream_t s, const c128* A, long strideA, c128* Ainv, lon
 }
 
 // ---------------------------------------------------------------------------------------------
-// Register-resident Gauss-Jordan / LU for 16 < N <= 32 (a matrix per warp was slower there: 27 x 27
-// in a warp's registers leaves too few warps an SM).  One CTA of 64 C threads per matrix (C = 2
-// column classes); thread t holds row i = t % 64 and the columns j = h + C q of class h = t / 64 in registers (q < QMAX), so a step
-// touches shared memory only for the pivot column, the pivot row and the row that moves in the
-// interchange.
+// Register-resident Gauss-Jordan / LU for 16 < N <= 32, and for the inverse of few matrices of N > 12
+// (a matrix per warp takes longer there: 27 x 27 in a warp's registers leaves too few warps an SM,
+// and one matrix of 16 x 16 waits on its own chain).  One CTA of four warps per matrix: lane i holds
+// row i and warp h the columns j = h + 4 q of it, in registers (q < QMAX), so a step touches shared
+// memory only for the pivot column, the pivot row and the row that moves in the interchange.
 // Step k: every warp finds the pivot p (first max |re|+|im| in column k, rows k..N-1, as izamax)
 // from the column buffer; the owners of row p write it as it stands with 1 in column k, the owners
 // of row k write the old row k; after one barrier every row i != k subtracts g_i times the pivot
@@ -328,26 +329,29 @@ void launch_gj_warp(cudaStream_t s, const c128* A, long strideA, c128* Ainv, lon
 // rows below k are eliminated (plain LU, the same U diagonal).  The row interchanges permute the
 // columns of the in-place inverse; they are undone on the way out (columns swapped in reverse step
 // order).  Two barriers a step.
+// Bound by the chain of a step (pivot search, reciprocal, two barriers); with 89 registers five CTAs
+// an SM overlap theirs.  Rows 0..63 on two column classes (half the lanes without a row, 164
+// registers, three CTAs) took 139.7 us for the inverses of 1024 matrices of N = 32 and 41.1 for 64
+// of them; this form 91.1 and 32.9.
 // ---------------------------------------------------------------------------------------------
-template <int QMAX, int C, bool INVERT>
-__global__ void __launch_bounds__(64 * C, 3) gj_reg_kernel(const c128* __restrict__ A,
-                                                               long strideA,
-                                                               c128* __restrict__ Ainv,
-                                                               long strideInv,
-                                                               c128* __restrict__ ovlp, int N,
-                                                               c128 post_scale, c128 post_add) {
-  __shared__ c128 rowbuf[64];     // pivot row, column k = 1
-  __shared__ c128 kbuf[64];       // old row k (moves to row p)
-  __shared__ c128 colbuf[2][64];  // column k of every row at step k (buffer k & 1)
-  __shared__ c128 piv_val[64];
-  __shared__ int perm[64];
-  __shared__ int pos[64];
+constexpr int GR_C = 4;  // column classes: warps of a CTA
+
+template <int QMAX, bool INVERT>
+__global__ void __launch_bounds__(32 * GR_C, QMAX <= 4 ? 6 : 5)
+    gj_reg_kernel(const c128* __restrict__ A, long strideA, c128* __restrict__ Ainv, long strideInv,
+                  c128* __restrict__ ovlp, int N, c128 post_scale, c128 post_add) {
+  constexpr int C = GR_C;
+  __shared__ c128 rowbuf[32];     // pivot row, column k = 1
+  __shared__ c128 kbuf[32];       // old row k (moves to row p)
+  __shared__ c128 colbuf[2][32];  // column k of every row at step k (buffer k & 1)
+  __shared__ c128 piv_val[32];
+  __shared__ int perm[32];
+  __shared__ int pos[32];
   __shared__ int s_singular;
 
   const int t = threadIdx.x;
-  const int i = t & 63;
-  const int h = t >> 6;  // column class: columns j = h + C q
-  const int lane = t & 31;
+  const int i = t & 31;
+  const int h = t >> 5;  // column class: columns j = h + C q
   const bool row_ok = i < N;
   const long w = blockIdx.x;
   const c128* Aw = A + w * strideA;
@@ -369,21 +373,16 @@ __global__ void __launch_bounds__(64 * C, 3) gj_reg_kernel(const c128* __restric
     const c128* col = colbuf[k & 1];
     // pivot: first max |re|+|im| in column k, rows k..N-1.  Non-negative doubles order as their
     // bit patterns, so the maximum is two warp max-reductions (high, then low word); NaN and rows
-    // outside k..N-1 take key 0.  The first row holding the maximum comes from two ballots.
-    const int r0 = k + lane, r1 = k + lane + 32;
-    const double v0 = r0 < N ? cabs1(col[r0]) : 0.0;
-    const double v1 = r1 < N ? cabs1(col[r1]) : 0.0;
-    const unsigned long long k0 = (v0 == v0) ? static_cast<unsigned long long>(__double_as_longlong(v0)) : 0ull;
-    const unsigned long long k1 = (v1 == v1) ? static_cast<unsigned long long>(__double_as_longlong(v1)) : 0ull;
-    const unsigned long long kl = k1 > k0 ? k1 : k0;
+    // outside k..N-1 take key 0.  The first row holding the maximum comes from a ballot.
+    const bool cand = row_ok && i >= k;
+    const double v = cand ? cabs1(col[i]) : 0.0;
+    const unsigned long long kl = (v == v) ? static_cast<unsigned long long>(__double_as_longlong(v)) : 0ull;
     const unsigned mhi = __reduce_max_sync(0xffffffffu, unsigned(kl >> 32));
     const unsigned mlo = __reduce_max_sync(0xffffffffu, unsigned(kl >> 32) == mhi ? unsigned(kl) : 0u);
     const unsigned long long kmax = (static_cast<unsigned long long>(mhi) << 32) | mlo;
     const bool zero = (kmax == 0ull);
-    const unsigned b0 = __ballot_sync(0xffffffffu, r0 < N && k0 == kmax);
-    const unsigned b1 = __ballot_sync(0xffffffffu, r1 < N && k1 == kmax);
-    // a zero (or NaN) column: zero pivot at row k, no interchange
-    const int p = zero ? k : (b0 ? k + __ffs(b0) - 1 : k + 32 + __ffs(b1) - 1);
+    // a zero (or NaN) column: every candidate ties, so zero pivot at row k, no interchange
+    const int p = __ffs(__ballot_sync(0xffffffffu, cand && kl == kmax)) - 1;
     const c128 piv = col[p];
     // 1/pivot = conj(pivot) / |pivot|^2
     const double rden = 1.0 / (piv.x * piv.x + piv.y * piv.y);
@@ -462,8 +461,6 @@ __global__ void __launch_bounds__(64 * C, 3) gj_reg_kernel(const c128* __restric
     }                                       \
     break;
         GR_CASE(0) GR_CASE(1) GR_CASE(2) GR_CASE(3) GR_CASE(4) GR_CASE(5) GR_CASE(6) GR_CASE(7)
-        GR_CASE(8) GR_CASE(9) GR_CASE(10) GR_CASE(11) GR_CASE(12) GR_CASE(13) GR_CASE(14)
-        GR_CASE(15)
 #undef GR_CASE
         default:
           break;
@@ -516,17 +513,6 @@ __global__ void __launch_bounds__(64 * C, 3) gj_reg_kernel(const c128* __restric
       }
     }
   }
-}
-
-template <int QMAX, int C>
-void launch_gj_reg(cudaStream_t s, const c128* A, long strideA, c128* Ainv, long strideInv,
-                   c128* ovlp, int W, int N, bool invert, c128 post_scale, c128 post_add) {
-  if (invert)
-    gj_reg_kernel<QMAX, C, true><<<W, 64 * C, 0, s>>>(A, strideA, Ainv, strideInv, ovlp, N,
-                                                      post_scale, post_add);
-  else
-    gj_reg_kernel<QMAX, C, false><<<W, 64 * C, 0, s>>>(A, strideA, nullptr, 0, ovlp, N,
-                                                       post_scale, post_add);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -756,11 +742,23 @@ int batched_logdet_inverse(cudaStream_t s, const c128* A, long strideA, c128* Ai
     launch_gj_warp<G, NC>(s, A, strideA, Ainv, strideInv, ovlp, W, N, invert, post_scale, post_add); \
     return launch_status("gj_warp_kernel"); \
   }
-    GJ_WARP(4, 4) GJ_WARP(8, 8) GJ_WARP(16, 12) GJ_WARP(16, 16)
+    GJ_WARP(4, 4) GJ_WARP(8, 8) GJ_WARP(16, 12)
+    // up to two matrices an SM the inverse takes 16.5 us by a CTA each and 20.6 by a warp (N = 16);
+    // 1024 of them 41 (as the CTA form then was) and 21.2.  The LU alone: 18.6 either way.
+    if (N <= 16 && invert && W <= 2 * NUM_SMS) {
+      gj_reg_kernel<4, true><<<W, 32 * GR_C, 0, s>>>(A, strideA, Ainv, strideInv, ovlp, N,
+                                                     post_scale, post_add);
+      return launch_status("gj_reg_kernel");
+    }
+    GJ_WARP(16, 16)
 #undef GJ_WARP
     if (N <= 32) {
-      launch_gj_reg<16, 2>(s, A, strideA, Ainv, strideInv, ovlp, W, N, invert, post_scale,
-                           post_add);
+      if (invert)
+        gj_reg_kernel<8, true><<<W, 32 * GR_C, 0, s>>>(A, strideA, Ainv, strideInv, ovlp, N,
+                                                       post_scale, post_add);
+      else
+        gj_reg_kernel<8, false><<<W, 32 * GR_C, 0, s>>>(A, strideA, nullptr, 0, ovlp, N, post_scale,
+                                                        post_add);
       return launch_status("gj_reg_kernel");
     }
     const size_t smem = gb_smem(N);

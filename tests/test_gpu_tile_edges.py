@@ -14,28 +14,37 @@ EPS = 2.0 ** -53
 
 @pytest.mark.parametrize("N", [1, 3, 4, 5, 8, 9, 12, 13, 16, 17, 20, 21, 24, 28, 29, 32, 33, 40, 41,
                                50, 57, 63, 64, 65])
-@pytest.mark.parametrize("W", [1, 37])
+@pytest.mark.parametrize("W", [1, 37, 300])
 def test_inverse_logdet(cuda, N, W):
+    """Inverses and log determinants.  A matrix with a zero first column is singular exactly: its
+    inverse is zero, and its log determinant takes the smallest number in the zero pivot's place and
+    goes on with the rows and columns that remain."""
     from safire_b200 import afqmc as A
     rs = np.random.default_rng(N)
     a = rand_c(rs, W, N, N)
     a[:, np.arange(N), np.arange(N)] *= 1e-3  # pivoting matters
-    if N > 1:
-        a[W - 1, :, N - 1] = a[W - 1, :, 0]   # singular to rounding: checked apart
     d_inv = torch.zeros((W, N, N), dtype=torch.complex128, device=cuda)
     d_log = torch.zeros(W, dtype=torch.complex128, device=cuda)
     A.det_ops.inverse_logdet(to_dev(a), d_inv, d_log)
     inv, log = to_host(d_inv), to_host(d_log)
-    for w in range(W if N == 1 else W - 1):
+    for w in range(W):
         cond = np.linalg.cond(a[w])
         assert np.linalg.norm(inv[w] @ a[w] - np.eye(N), 2) < 50 * N * EPS * cond
         sign, la = np.linalg.slogdet(a[w])
         assert abs(log[w].real - la) < 50 * N * EPS * cond
         assert abs(np.exp(1j * log[w].imag) - sign) < 50 * N * EPS * cond
-    # a zero column is singular exactly: a zero inverse
     a[:, :, 0] = 0.0
+    d_log.zero_()
     A.det_ops.inverse_logdet(to_dev(a), d_inv, d_log)
     assert np.all(to_host(d_inv) == 0)
+    log = to_host(d_log)
+    for w in range(W):
+        rest = a[w, 1:, 1:]
+        cond = np.linalg.cond(rest) if N > 1 else 1.0
+        sign, la = np.linalg.slogdet(rest)
+        tol = 50 * N * EPS * cond + 1e-12  # the logarithm of the smallest number, -708, has 1e-13
+        assert abs(log[w].real - np.log(np.finfo(float).tiny) - la) < tol
+        assert abs(np.exp(1j * log[w].imag) - sign) < tol
 
 
 @pytest.mark.parametrize("M,N", [(9, 1), (8, 8), (30, 9), (40, 31), (64, 32), (70, 50), (80, 64),
