@@ -264,13 +264,16 @@ def test_phmsd_energy_index_groups(cuda, nup, ndn, nocc, nvirt, Nc, ndet):
     assert np.all(np.abs(out[1] - out[0]) < 5e-5 * scale)
 
 
-@pytest.mark.parametrize("M,N,Nc,W", [(40, 13, 8, 1), (72, 32, 44, 130), (104, 50, 264, 33), (136, 50, 24, 7)])
+@pytest.mark.parametrize("M,N,Nc,W", [(40, 13, 8, 1), (64, 32, 16, 9), (72, 32, 44, 130), (128, 32, 8, 5),
+                                      (104, 50, 264, 33), (136, 50, 24, 7), (256, 32, 8, 2),
+                                      (168, 50, 16, 3)])
 @pytest.mark.parametrize("fmt", [1, 2])  # TF32, FP16 split
 def test_mixed_vbias_ranges(cuda, M, N, Nc, W, fmt):
     """The force bias summed over ranges of its K = N M (one, and several) in mixed precision, against
-    complex128.  Operands keep 22 bits, and a running sum in FP32 loses up to 2^-23 of itself with
-    each MMA of 16 elements; it is about the size of a result, of which the largest of the deviations
-    is taken as eight."""
+    complex128, at the edges of the blocks that split its rows (2048, 4096 and 8192 values).  Operands
+    keep 22 bits, and a range's running sum in FP32 loses up to 2^-23 of itself with each MMA (16
+    elements in FP16, 8 in TF32); it is about the size of a result, of which the largest of the
+    deviations is taken as eight."""
     from safire_b200 import afqmc as A
     rs = np.random.default_rng(M)
     Nc -= Nc % 8 if fmt == 2 else 0  # the FP16 split takes multiples of 8
@@ -283,7 +286,9 @@ def test_mixed_vbias_ranges(cuda, M, N, Nc, W, fmt):
     ham.vbias(G, r, 0.01)
     assert ham.device_error_flag() == 0
     v, r = to_host(v), to_host(r)
-    bound = 8 * (2.0 ** -21 + N * M / 16 * 2.0 ** -23)
+    step, K = (8, N * M) if fmt == 2 else (4, N * M)
+    S = next((c for c in range(16, 1, -1) if K % (c * step) == 0 and K // c >= 512), 1)
+    bound = 8 * (2.0 ** -21 + K / S / (2 * step) * 2.0 ** -23)
     assert np.max(np.abs(v - r)) < bound * np.sqrt(np.mean(np.abs(r) ** 2))
 
 
