@@ -108,6 +108,10 @@ __global__ void __launch_bounds__(XT_THREADS, 1) exchange_tc_kernel(const __grid
   constexpr int NA = NSPLIT == 3 ? 2 : 1;      // planes of each part
   constexpr int NCOL = SA == 64 ? 56 : SA;     // accumulator columns a thread holds per walker
   constexpr int A_TILE = X_ROWS * XBK * 4;
+  // The pairs a < b once, or all of them: half the lanes' accesses to shared memory against a
+  // comparison of each lane's a with every b.  Measured (M = 104, N = 40, 400 vectors, 1024 walkers),
+  // the triangle and all pairs: FP16 3.01 and 3.22 ms, TF32 3.55 and 3.15.
+  constexpr bool ALL_PAIRS = !F16;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -271,8 +275,8 @@ __global__ void __launch_bounds__(XT_THREADS, 1) exchange_tc_kernel(const __grid
 #pragma unroll 1
       for (int wl = 0; wl < nw; ++wl) {
         const int w = wp * p.NW + wl;
-        // row a of the block (columns b) into registers, and its lower triangle into the staging
-        // block, from which the rows above read it as their column
+        // row a of the block (columns b) into registers, and its lower triangle (or the whole row)
+        // into the staging block, from which the rows above (or all) read it as their column
         float vr[NCOL], vi[NCOL];
         {
           const uint32_t cr = trow + uint32_t(wl * p.SB), ci_ = cr + uint32_t(ncols);
@@ -291,7 +295,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) exchange_tc_kernel(const __grid
         if (valid) {
 #pragma unroll
           for (int b = 0; b < NCOL; ++b)
-            if (b <= a) row[b] = make_float2(vr[b], vi[b]);
+            if (ALL_PAIRS ? b < N : b <= a) row[b] = make_float2(vr[b], vi[b]);
         }
         // the running sum this thread adds to, fetched now so its latency hides behind the loop
         double* out = nullptr;
@@ -301,25 +305,27 @@ __global__ void __launch_bounds__(XT_THREADS, 1) exchange_tc_kernel(const __grid
           old = *out;
         }
         named_bar(1, 128);
-        // x = T[a][a]^2 + 2 sum_{b > a} T[a][b] T[b][a];  tr = T[a][a].  The sum over b runs in
-        // FP32 with four independent accumulator pairs; the partial sums are widened to FP64 for
+        // x = T[a][a]^2 + 2 sum_{b > a} T[a][b] T[b][a], or sum_b T[a][b] T[b][a] where the
+        // block is whole;  tr = T[a][a].  The sum over b runs in FP32 with four independent accumulator pairs; the partial sums are widened to FP64 for
         // every later sum.
         double v4[4] = {0.0, 0.0, 0.0, 0.0};
         if (valid) {
           float xr[4] = {0.f, 0.f, 0.f, 0.f}, xi[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int b = 0; b < NCOL; ++b)
-            if (b < N && b > a) {
+            if (b < N && (ALL_PAIRS || b > a)) {
               const float2 u = col[b * PITCH];  // T[b][a]
               xr[b & 3] = fmaf(vr[b], u.x, fmaf(-vi[b], u.y, xr[b & 3]));
               xi[b & 3] = fmaf(vr[b], u.y, fmaf(vi[b], u.x, xi[b & 3]));
             }
           const float2 d = row[a];
           const double dr = d.x, di = d.y;
-          v4[0] = 2.0 * ((double(xr[0]) + double(xr[1])) + (double(xr[2]) + double(xr[3]))) +
-                  (dr * dr - di * di);
-          v4[1] = 2.0 * ((double(xi[0]) + double(xi[1])) + (double(xi[2]) + double(xi[3]))) +
-                  2.0 * dr * di;
+          v4[0] = (double(xr[0]) + double(xr[1])) + (double(xr[2]) + double(xr[3]));
+          v4[1] = (double(xi[0]) + double(xi[1])) + (double(xi[2]) + double(xi[3]));
+          if (!ALL_PAIRS) {
+            v4[0] = 2.0 * v4[0] + (dr * dr - di * di);
+            v4[1] = 2.0 * v4[1] + 2.0 * dr * di;
+          }
           v4[2] = dr;
           v4[3] = di;
         }
