@@ -410,7 +410,7 @@ extern "C" int afqmc_propagate(const afqmc_c128* P1, const afqmc_c128* V, afqmc_
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   Scratch w;
   const size_t one = size_t(W) * M * N;
-  if (!taylor_c128_fits(M, N)) AFQMC_TRY(w.get(sizeof(c128) * one * 3, s));
+  if (!taylor_c128_fits(W, M, N)) AFQMC_TRY(w.get(sizeof(c128) * one * 3, s));
   c128* b = (c128*)w.p;
   return propagate(s, P1, false, (const c128*)V, long(M) * M, (c128*)S, ldS, W, M, N, order, b,
                    b + one, b + 2 * one);

@@ -852,7 +852,7 @@ int mixed_density_matrix(cudaStream_t s, const c128* PsiT, const c128* S, long l
 int propagate(cudaStream_t s, const void* P1, bool p1_real, const c128* V, long strideV, c128* S,
               long ldS, int W, int M, int N, int order, c128* work1, c128* work2, c128* work3) {
   if (N == 0 || W == 0) return AFQMC_OK;
-  if (taylor_c128_fits(M, N))
+  if (taylor_c128_fits(W, M, N))
     return taylor_c128(s, P1, p1_real, V, strideV, S, ldS, W, M, N, order);
   const long sMN = long(M) * N;
   // T0 = P1 * S into work2, and the running sum TMN = T0 into work1

@@ -26,14 +26,14 @@ int mixed_density_matrix(cudaStream_t s, const c128* PsiT, const c128* S, long l
                          c128* work_NM, c128 post_scale, c128 post_add,
                          const double* PsiT_r = nullptr);
 
-// the same in one launch, for the sizes that fit an SM (taylor_fp64.cu)
-bool taylor_c128_fits(int M, int N);
-int taylor_c128(cudaStream_t s, const void* P1, bool p1_real, const c128* V, long strideV, c128* S,
-                long ldS, int W, int M, int N, int order);
-
-// S <- P1 exp_T(i V) P1 S.  work1..3: [W][M][N] each (not touched where taylor_c128 fits).
+// S <- P1 exp_T(i V) P1 S.  work1..3: [W][M][N] each (not touched where taylor_c128_fits).
 int propagate(cudaStream_t s, const void* P1, bool p1_real, const c128* V, long strideV, c128* S,
               long ldS, int W, int M, int N, int order, c128* work1, c128* work2, c128* work3);
+
+// the same in one launch (taylor_fp64.cu), and whether that is possible and faster
+bool taylor_c128_fits(int W, int M, int N);
+int taylor_c128(cudaStream_t s, const void* P1, bool p1_real, const c128* V, long strideV, c128* S,
+                long ldS, int W, int M, int N, int order);
 
 // det_ops::orthogonalize: S_w <- Q_w diag(sign(Re R_ii)), logdetR[w] += sum log(|R_ii|).
 // work: [W*M*N + 2*W*N*N] complex, or nullptr to take it from the stream-ordered allocator.

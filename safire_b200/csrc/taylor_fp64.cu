@@ -12,7 +12,8 @@
 // walkers an SM the latency of one walker's chain.  Whole steps with the launches and with this:
 // M = 32, N = 8, 64 walkers 102 -> 77 us; M = 19, N = 3, 1536 walkers, two spins 619 -> 511 us;
 // M = 100, N = 25, 256 walkers 708 -> 640 us.  Past N = 32 or M = 128 the accumulators and T, R
-// no longer fit beside enough warps, and the products are large enough for GEMM launches.
+// no longer fit beside enough warps, and the products are large enough for GEMM launches; where these
+// are faster below that, taylor_c128_fits tells.
 #include <type_traits>
 
 #include "detops.cuh"
@@ -239,8 +240,21 @@ int run_tn(cudaStream_t s, const void* P1, bool p1_real, const c128* V, long str
 
 }  // namespace
 
-bool taylor_c128_fits(int M, int N) {
-  return N >= 1 && N <= 32 && M >= 1 && M <= 128 && smem_bytes(M, (N + 7) / 8) <= 227 * 1024;
+// M <= 64 (a strip per warp, two CTAs an SM where the accumulators are small): always.  Above that
+// one CTA fits an SM by its registers and takes about the same time whatever the number of walkers, so
+// with wide accumulators (N > 16) it depends on how many SMs the last wave leaves idle.  GEMM launches
+// over this form, times of order 6 (1 to 1024 walkers; fill = W / 148 over the waves):
+//   M = 48 to 64: 1.2 to 3.1 at every N from 32 walkers on
+//   N <= 16, M = 65 to 128: 0.9 to 2.7 from 32 walkers on
+//   N = 17..24: 0.86 to 1.15 at 32 walkers (fill 0.22), 1.2 at 60, 0.92 to 1.6 from 140 on
+//   N = 25..32: M = 80 and 96: 0.77 at 149 walkers (0.50) and 300 (0.68), 0.83 at 445 (0.75), 0.84 to
+//     0.89 at 600 (0.81), 1.03 at 256 (0.86), 1.12 at 296 (1.0), 0.92 to 0.95 at 1024 (0.99);
+//     M = 100 to 128: 0.95 at 149, 0.97 to 1.02 at 200 (0.68) and 300, 1.27 at 296, 1.13 at 1024
+bool taylor_c128_fits(int W, int M, int N) {
+  if (N < 1 || N > 32 || M < 1 || M > 128 || smem_bytes(M, (N + 7) / 8) > 227 * 1024) return false;
+  if (M <= 64 || N <= 16) return true;
+  const double fill = double(W) / (double(NUM_SMS) * ceil_div(W, NUM_SMS));
+  return fill >= (N <= 24 ? 0.3 : M <= 96 ? 0.85 : 0.65);
 }
 
 int taylor_c128(cudaStream_t s, const void* P1, bool p1_real, const c128* V, long strideV, c128* S,

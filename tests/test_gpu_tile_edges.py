@@ -69,10 +69,10 @@ def test_orthogonalize(cuda, M, N):
 @pytest.mark.parametrize("M,N", [(5, 1), (19, 3), (32, 8), (32, 32), (33, 9), (64, 16), (65, 24),
                                  (101, 23), (128, 32), (129, 8), (70, 33)])
 @pytest.mark.parametrize("order", [0, 1, 6])
-def test_propagate(cuda, M, N, order):
+@pytest.mark.parametrize("W", [3, 140])  # N > 16, M > 64: GEMM launches, and one launch for an SM each
+def test_propagate(cuda, M, N, order, W):
     from safire_b200 import afqmc as A
     rs = np.random.default_rng(M + N)
-    W = 3
     P1 = np.eye(M) + rand_c(rs, M, M, scale=0.1 / np.sqrt(M))
     V = rand_c(rs, W, M, M, scale=0.5 / np.sqrt(M))
     S = rand_c(rs, W, M, N)
