@@ -62,6 +62,7 @@ int dalloc(T** p, size_t n) {
   if (n == 0) return AFQMC_OK;
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), n * sizeof(T));
   if (e != cudaSuccess) {
+    cudaGetLastError();
     set_error_detail("cudaMalloc of %zu bytes failed: %s", n * sizeof(T), cudaGetErrorString(e));
     return AFQMC_ERR_ALLOC;
   }
@@ -274,6 +275,7 @@ struct Scratch {
     retain_pool_memory();
     cudaError_t e = cudaMallocAsync(&p, bytes, st);
     if (e != cudaSuccess) {
+      cudaGetLastError();
       set_error_detail("cudaMallocAsync(%zu) failed: %s", bytes, cudaGetErrorString(e));
       p = nullptr;
       return AFQMC_ERR_ALLOC;

@@ -46,10 +46,13 @@ __host__ __device__ __forceinline__ c128 cexp(c128 a) {
 void set_error_detail(const char* fmt, ...);
 const char* error_detail();
 
+// A failed runtime call also stays behind as the thread's last error, where the next launch, ours or
+// the caller's, would find it: it is taken out once it is reported.
 #define AFQMC_CUDA_TRY(expr)                                                               \
   do {                                                                                     \
     cudaError_t e_ = (expr);                                                               \
     if (e_ != cudaSuccess) {                                                               \
+      cudaGetLastError();                                                                  \
       ::afqmc::set_error_detail("%s:%d %s: %s", __FILE__, __LINE__, #expr,                 \
                                 cudaGetErrorString(e_));                                   \
       return AFQMC_ERR_CUDA;                                                               \

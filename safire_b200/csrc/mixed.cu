@@ -619,6 +619,7 @@ int alloc_planes(Planes& P, int nplanes, long batch, long rows, long k, int esiz
   for (int q = 0; q < nplanes; ++q) {
     cudaError_t e = cudaMalloc(&P.p[q], size_t(esize) * P.elems());
     if (e != cudaSuccess) {
+      cudaGetLastError();
       set_error_detail("alloc_planes: %s", cudaGetErrorString(e));
       return AFQMC_ERR_ALLOC;
     }

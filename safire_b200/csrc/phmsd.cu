@@ -2220,6 +2220,7 @@ extern "C" int afqmc_phmsd_set_hamiltonian(afqmc_phmsd h, const double* Likn, in
   c128 *hd = nullptr, *tmp = nullptr;
   int st = AFQMC_OK;
   auto fail = [&](int code) {
+    cudaGetLastError();
     cudaFree(L);
     cudaFree(hd);
     cudaFree(tmp);
@@ -2283,6 +2284,7 @@ namespace {
 
 int scratch_alloc(c128** p, size_t n) {
   if (cudaMalloc(p, sizeof(c128) * (n ? n : 1)) != cudaSuccess) {
+    cudaGetLastError();
     set_error_detail("PHMSD scratch: out of device memory (%zu bytes)", sizeof(c128) * n);
     return AFQMC_ERR_ALLOC;
   }
@@ -2694,7 +2696,6 @@ extern "C" int afqmc_phmsd_density_matrix(afqmc_phmsd h, const afqmc_c128* wbuf,
     Wb = std::min(Wb, SETTLED);
   int st = phmsd_core_scratch(h, Wb);
   if (st == AFQMC_ERR_ALLOC && block <= 0 && Wb > SETTLED) {
-    cudaGetLastError();
     Wb = SETTLED;
     st = phmsd_core_scratch(h, Wb);
   }

@@ -140,6 +140,7 @@ __global__ void thc_xx_kernel(const double* __restrict__ X, int M, int nu, doubl
 
 int thc_cuda(cudaError_t e, const char* what) {
   if (e == cudaSuccess) return AFQMC_OK;
+  cudaGetLastError();
   set_error_detail("%s: %s", what, cudaGetErrorString(e));
   return e == cudaErrorMemoryAllocation ? AFQMC_ERR_ALLOC : AFQMC_ERR_CUDA;
 }

@@ -85,8 +85,8 @@ def test_singular_inverse_is_zero(cuda):
 
 @pytest.mark.parametrize("N", [1, 2, 7, 8, 9, 16, 17, 32, 33, 50, 52, 53, 64, 65, 70])
 def test_random_inverse_logdet_sizes(cuda, N):
-    """Every size class of the register-resident kernel (N <= 64) and the shared-memory kernel
-    (N > 64): inverse and accumulated log det against the oracle's getrf/getri."""
+    """Every size class (a group of lanes to N = 16, a CTA's registers to 32, panels in shared memory
+    to 64, one array there above): inverse and accumulated log det against the oracle's getrf/getri."""
     A = _A()
     rs = np.random.default_rng(100 + N)
     W = 5

@@ -165,6 +165,17 @@ def test_phmsd_density_matrix_captured(cuda, W):
         assert np.array_equal(to_host(G), want), first
 
 
+def test_failed_call_leaves_no_error(cuda):
+    """A call that the runtime refuses (a block sum of 121 electrons passes an SM's shared memory)
+    reports it, and neither a later call nor the caller's own runtime finds the error again."""
+    from safire_b200 import afqmc as A
+    from safire_b200.capi import AfqmcError
+    with pytest.raises(AfqmcError):
+        _energy_call(122, 121, A.PREC_FP64)()
+    assert torch.isfinite(torch.ones(4, device=cuda).exp()).all()
+    assert np.all(np.isfinite(to_host(_energy_call(24, 5, A.PREC_FP64)()).view(float)))
+
+
 def _energy_call(M, N, precision):
     from safire_b200 import afqmc as A
     rs = np.random.default_rng(N)
