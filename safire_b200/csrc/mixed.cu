@@ -123,10 +123,6 @@ __device__ __forceinline__ void tc_tile(long t, int MT, int NT, int order, int& 
   }
 }
 
-// Epilogue of a symmetric vHS tile (BN = 128 columns = 8 x 16 (i, k) pairs) for one walker row:
-// each value goes to V[w][i][k] (i <= k) and V[w][k][i] (i < k), the real then the imaginary
-// part, so that a thread holds a whole 8 x 16 block (128 registers) and writes rows of 16 (direct)
-// and 8 (mirrored) consecutive floats.
 // 32 bytes to a 32-byte boundary: a whole sector
 __device__ __forceinline__ void store_sector(void* dst, const uint32_t (&v)[8]) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(v[0]), "r"(v[1]),
@@ -194,6 +190,10 @@ __device__ __forceinline__ void store_run16(__half* hi, __half* lo, long idx, co
   }
 }
 
+// Epilogue of a symmetric vHS tile (BN = 128 columns = 8 x 16 (i, k) pairs) for one walker row:
+// each value goes to V[w][i][k] (i <= k) and V[w][k][i] (i < k), the real then the imaginary
+// part, so that a thread holds a whole 8 x 16 block (128 registers) and writes rows of 16 (direct)
+// and 8 (mirrored) consecutive values.
 __device__ __forceinline__ void vhs_sym_epilogue(const TcParams& p, uint32_t trow, int row, int nt,
                                                  uint64_t* acc_free) {
   int ab, cb;

@@ -6,7 +6,7 @@ import torch
 
 from oracle import phmsd as P
 from tests.golden import phmsd_golden as g
-from tests.gpu_helpers import rel_err, to_dev, to_host
+from tests.gpu_helpers import rand_c, rel_err, to_dev, to_host
 
 pytestmark = pytest.mark.gpu
 
@@ -151,6 +151,55 @@ def test_phmsd_energy_vs_oracle(cuda, M, nup, ndn, Nc, nocc, nvirt, ndet, W, blo
     d = to_host(ov) - ovo
     d = d.real + 1j * ((d.imag + np.pi) % (2 * np.pi) - np.pi)
     assert np.max(np.abs(d)) < 1e-10
+
+
+@pytest.mark.parametrize("M,nup,ndn,Nc,nocc,nvirt,ndet,level", [
+    (24, 9, 9, 11, 8, 9, 120, 8),      # up to eight holes of a spin; complex64 rows (M = 0 mod 8)
+    (22, 9, 8, 10, 8, 8, 80, 8),       # the same with complex128 rows
+    (80, 38, 37, 7, 8, 40, 40, 4),     # four holes; tables of eight vectors pass 225 KB, of four 110
+    (96, 48, 46, 5, 10, 40, 30, 4),    # tables of four vectors pass 110 KB in complex64, 200 in complex128
+    (96, 48, 46, 5, 10, 40, 30, 6)])   # ... with more than four holes
+def test_phmsd_forms_vs_oracle(cuda, M, nup, ndn, Nc, nocc, nvirt, ndet, level):
+    """The forms of the excited determinants' terms (five to eight holes in kernels of their own;
+    eight, four or one Cholesky vector to a CTA) and the density matrix, against the oracle.  All
+    determinants weigh about the same, so that those of many holes show.  Mixed energies: a block's
+    sums round up to 2 n = 16 times in single precision, each amplified by the condition of the
+    excitation blocks whose inverses enter, taken in the mean over the determinants."""
+    from safire_b200 import afqmc as A
+    from safire_b200.synth import make_hamiltonian, make_phmsd_trial
+    h1, Likn = make_hamiltonian(M, Nc, 0.9, seed=M)
+    _, C = np.linalg.eigh(h1)
+    t = make_phmsd_trial(M, nup, ndn, C, nocc=nocc, nvirt=nvirt, ndet=ndet, seed=M, max_level=level)
+    rs = np.random.default_rng(M + 2)
+    t.coef = rs.uniform(0.5, 1.0, ndet).astype(complex)
+    assert level < 8 or {5, 6, 7, 8} <= set(t.exc[0])
+    hij, W = h1[None].astype(complex), 3
+    S = [rand_c(rs, W, M, n, scale=1 / np.sqrt(M)) for n in (nup, ndn)]
+    H = P.ActiveSpaceHamiltonian(t, Likn[None], hij, 0.3)
+    Eo, ovo = P.phmsd_energy(t, H, *S)
+    share, cond = t.coef[:, None] * np.ones((1, W), complex), np.zeros((ndet, W))
+    for s, det in ((0, t.det_up), (1, t.det_dn)):
+        Q = P.mixed_density_matrix_for_woodbury(t.orbmat[s], S[s], t.refc[s])[2]
+        share *= P.excitation_overlaps(t, s, Q)[det]
+        cond += np.array([np.ones(W)] + [np.linalg.cond(Q[:, e[n:]][:, :, e[:n]])
+                                         for n in sorted(t.exc[s]) for e in t.exc[s][n]])[det]
+    amp = np.max(np.sum(np.abs(share) * cond, 0) / np.abs(np.sum(share, 0)))
+    wbuf = to_dev(np.concatenate([s.reshape(W, -1) for s in S], 1))
+    ph = A.PHMSD(t)
+    ph.set_hamiltonian(Likn[None], hij, 0.3)
+    E = torch.zeros((W, 3), dtype=torch.complex128, device=cuda)
+    ov = torch.zeros(W, dtype=torch.complex128, device=cuda)
+    for prec, tol in ((A.PREC_FP64, 1e-10), (A.PREC_MIXED, 16 * 2.0 ** -24 * amp)):
+        ph.set_precision(prec)
+        ph.Energy(wbuf, E, ov)
+        errs = np.array([rel_err(to_host(E)[:, q], Eo[:, q]) for q in range(3)])
+        assert np.all(errs < tol), (prec, errs, tol)
+        d = to_host(ov) - ovo
+        assert np.max(np.abs(d.real + 1j * ((d.imag + np.pi) % (2 * np.pi) - np.pi))) < 1e-10
+    G = torch.zeros((W, sum(o.shape[0] for o in t.orbmat), M), dtype=torch.complex128, device=cuda)
+    ph.MixedDensityMatrix(wbuf, G, ov)
+    Go, _ = P.phmsd_mixed_density_matrix(t, *S)
+    assert rel_err(to_host(G), Go) < 1e-10
 
 
 @pytest.mark.gpu
