@@ -82,18 +82,21 @@ double model_time(const Shape& sh, int m, int n, int k, bool a_real, bool b_real
 // 64 x 64 tiles fill the SMs twice over
 bool many_tiles(int m, long n) { return ceil_div(m, 64) * long(ceil_div(n, 64)) >= 2 * NUM_SMS; }
 
-// The shape for a single problem of few tiles: that of least time by the model, if it saves a tenth of
-// the fitted tiles' time.  K is split in two K tiles or more each, and not where there are many tiles.
-// On the problems above the choice is within 8.6% of the fastest shape in the mean, 35% at worst.  The
-// fitted tiles, with K split in eight K tiles or more, took 1.5 times as long: 1024 x 400 x 4160
-// (real B) in tiles of 64 x 40 is 160 CTAs, two on 12 of the SMs and one on the others (462 us, now
-// 335), and 1 x 4096 x 200 one warp an SM (27.5 us, now 11).
+// The shape for a single problem of few tiles: the fitted one, or that of least time by the model if it
+// saves a twentieth.  K is split in two K tiles or more each, and not where there are many tiles.  On
+// the problems above and 61 that the steps and energies of molecules and model systems pose, the choice
+// is within 8% of the fastest of all shapes in the mean, and never more than 1.5% slower than the
+// fitted shape alone, which took 1.36 times the fastest in the mean: 1024 x 400 x 4160 (real B) in
+// tiles of 64 x 40 is 160 CTAs, two on 12 of the SMs and one on the others (462 us; in 32 x 32 333),
+// and 1 x 4096 x 200 one warp an SM (27.5 us; in 16 x 8 11).  More widths than these four cost the host
+// time (0.4 us for four) and gain 1%.
 Shape least_time(Shape fit, int m, int n, int k, bool a_real, bool b_real) {
   const int ktiles = ceil_div(k, BK);
   const bool may_split = !many_tiles(m, n);
-  double least = 0.9 * model_time(fit, m, n, k, a_real, b_real);
+  double least = 0.95 * model_time(fit, m, n, k, a_real, b_real);
   for (int w = m >= 64 ? 4 : 1; w <= 8 && (w <= 2 || m > 4 * w); w *= 2)
-    for (int tn = 1; tn <= 8 && n > 8 * (tn - 1); ++tn)
+    for (const int tn : {1, 2, 4, 7}) {
+      if (n <= 8 * (tn - 1)) break;
       for (int c = 1; c <= 8 && (c == 1 || (may_split && ktiles >= 2 * c)); c *= 2) {
         const double t = model_time({w, tn, c}, m, n, k, a_real, b_real);
         if (t < least) {
@@ -101,24 +104,29 @@ Shape least_time(Shape fit, int m, int n, int k, bool a_real, bool b_real) {
           fit = {w, tn, c};
         }
       }
+    }
   return fit;
 }
 
 }  // namespace
 
-// The CTA shape: tiles fitted to m and n; where those of a batch are too few to give every SM one,
-// halved down to 8 strips in all (below that the operand loads bound a tile).  A single problem of few
-// tiles takes the shape of least time.
+// The CTA shape: tiles fitted to m and n; then, where those are too few to give every SM one, the K
+// range of a single problem split over a cluster of up to 8 CTAs (each keeping at least 8 K tiles),
+// and the tiles halved down to 8 strips in all (below that the operand loads bound a tile).  For a
+// single problem of few tiles the model looks for a faster one.
 Shape shape(int batch, int m, int n, int k, bool a_real, bool b_real) {
   Shape sh{fit_rows(m), fit_cols(n), 1};
   auto ctas = [&] { return long(ceil_div(m, 8 * sh.warps)) * ceil_div(n, 8 * sh.tn) * batch; };
-  if (batch == 1 && ctas() < 5 * NUM_SMS) return least_time(sh, m, n, k, a_real, b_real);
-  while (ctas() < NUM_SMS && sh.warps * sh.tn > 8) {
+  const bool few = batch == 1 && ctas() < 5 * NUM_SMS;
+  if (batch == 1 && ctas() < NUM_SMS)
+    sh.split = std::max(1, std::min({8, int(NUM_SMS / ctas()), ceil_div(k, BK) / 8}));
+  while (ctas() * sh.split < NUM_SMS && sh.warps * sh.tn > 8) {
     if (sh.tn >= sh.warps)
       sh.tn = (sh.tn + 1) / 2;
     else
       sh.warps = (sh.warps + 1) / 2;
   }
+  if (few) return least_time(sh, m, n, k, a_real, b_real);
   if (m > 65535l * 8 * sh.warps) sh.warps = 8;  // grid.y limit
   return sh;
 }
