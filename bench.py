@@ -479,9 +479,9 @@ def _roofline(sim, wl, W, prec, phases, args, torch, taylor_mode=1):
     peak = the dense rate of the MMA kind the kernel issues: the measured BF16 rate of
     MEASURED_PEAKS.json for the FP16 split (kind::f16 runs FP16 and BF16 at one rate), cuBLAS TF32
     at 8192^3 measured in this run for the TF32 split, cuBLAS DGEMM for complex128 (the file has
-    no TF32 or FP64 entry).  `mma_tflops` / `mma_frac` give the tensor work the kernels actually
-    issue (real Lnak, L and P1; three products per real product for the split), against the
-    same peak."""
+    no TF32 or FP64 entry).  `mma_tflops` / `mma_frac` give the products the kernels form on the
+    tensor cores (real Lnak, L and P1; three products per real product for the split), without the
+    padding of their tiles, against the same peak."""
     from safire_b200 import afqmc as A
     M, N, Nc = wl.M, wl.nup, wl.Nc
     order = 6
@@ -540,7 +540,8 @@ def _roofline(sim, wl, W, prec, phases, args, torch, taylor_mode=1):
         t_launch = x0.elapsed_time(x1) / reps
         del G, E
         kernel = f"exchange_tc_kernel<{args.exchange_split}> (fused EXX/EJ contraction)"
-        traffic, traffic_src = _EXCHANGE_TRAFFIC(W, Nc, N, M, 2 if f16 else 4)
+        traffic, traffic_src = _EXCHANGE_TRAFFIC(W, Nc, N, M, 2 if f16 else 4,
+                                                 sim.ham.get_tiles()[1])
     if top == "propagate" and prec == A.PREC_MIXED:
         traffic, traffic_src = _TAYLOR_TRAFFIC(W, M, N, taylor_mode)
     achieved = algo[top] / (t_launch / 1000) / 1e12
@@ -553,31 +554,34 @@ def _roofline(sim, wl, W, prec, phases, args, torch, taylor_mode=1):
             "mma_flops_per_launch": issued[top], "block_share_ms": block_share}
 
 
-def _EXCHANGE_TRAFFIC(W, Nc, N, M, esize=2):
-    """DRAM bytes per launch of exchange_tc_kernel<3>: ncu (dram__bytes_read.sum +
-    dram__bytes_write.sum) at the bench's 1024 walkers read 1.162 GB and wrote 53.9 MB with FP16
-    split planes (esize 2; 2.316 GB and 55.6 MB with TF32 planes).  The tile order keeps the Lnak
-    planes of 64 vector pairs in L2 while every walker pair passes, so the reads are the Lnak
-    planes once plus every walker's G planes once per 64-pair block, and the writes the two
-    complex sums per (walker, vector); other walker counts scale by that."""
+def _EXCHANGE_TRAFFIC(W, Nc, N, M, esize=2, pairs=64):
+    """DRAM bytes per launch of exchange_tc_kernel<64, 3>: ncu (dram__bytes_read.sum +
+    dram__bytes_write.sum) at the bench's 1024 walkers, by the bytes of a plane's element (2: FP16
+    split, 4: TF32) and the vector pairs per L2 block of the tile order.  The Lnak planes of a block
+    stay in L2 while every walker passes, so the reads are the Lnak planes once plus every walker's G
+    planes once per block, and the writes the two complex sums per (walker, vector); other sizes
+    scale by that."""
     src = "ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch at 1024 walkers"
-    if (W, Nc, N, M) == (1024, 1600, 50, 200):
-        return (1161931776 + 53940480 if esize == 2 else 2315739136 + 55630080), src
-    blocks = -(-((Nc + 1) // 2) // 64)
+    measured = {(2, 64): 1159181824 + 56070400, (2, 16): 4514687488 + 55389440,
+                (4, 64): 2309666816 + 55523328, (4, 16): 8353797120 + 56682496}
+    if (W, Nc, N, M) == (1024, 1600, 50, 200) and (esize, pairs) in measured:
+        return measured[esize, pairs], src
+    blocks = -(-((Nc + 1) // 2) // pairs)
     return (2 * Nc * N * M * esize + W * (4 * N * M * esize) * blocks + W * Nc * 32,
-            src + " scaled by the tile-order model to other walker counts")
+            src + " scaled by the tile-order model")
 
 
 def _TAYLOR_TRAFFIC(W, M, N, taylor_mode):
-    """DRAM bytes per launch of taylor_tc_kernel: ncu (dram__bytes_read.sum +
+    """DRAM bytes per launch of taylor_il_kernel: ncu (dram__bytes_read.sum +
     dram__bytes_write.sum) of the second launch at the bench's 1024 walkers, FP16 split with the
-    second accumulator (mode 4): 578.4 MB read, 626.5 MB written, against 574 MB of compulsory
-    traffic (V planes 328 MB and S planes 82 MB read once, S 164 MB written).  The excess writes
-    are the terms' planes and the FP32 running sum leaving L2.  Other walker counts scale with
-    the walkers."""
+    second accumulator (mode 4): 2.882 GB read, 1.111 GB written, against 587 MB of compulsory
+    traffic (V planes 341 MB, their rows padded to 208, and S planes 82 MB read once, S 164 MB
+    written).  Two walkers a CTA keep 296 V's of 333 KB in turn, which L2 does not hold over the six
+    terms; the excess writes are the terms' planes and the FP32 running sum leaving L2.  Other
+    walker counts scale with the walkers."""
     if (M, N) != (200, 50) or taylor_mode != 4:
         return None, None
-    return (578384640 + 626533888) * W // 1024, \
+    return (2882350080 + 1111400192) * W // 1024, \
         "ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch at 1024 walkers " \
         "(taylor mode 4), scaled by the walkers"
 
@@ -874,24 +878,28 @@ def run_phmsd(args):
     sim.restart()
     phases = _phases(sim)
     # the excited-determinant energy tables, per (walker, Cholesky index) and spin: the table
-    # products Y = t[:, r] QQ0^T (nel x nv x nel), U = t[holes, r] t (nh x nact x nel),
-    # Z = t[holes, r] Y (nh x nv x nel), then 3 n^3 + 6 n^2 + 3 n complex MACs per n-hole
-    # determinant (the closed-form sums of excited_terms); 8 flops per complex MAC
+    # products t[:, r] QQ0^T (nel x nv x nel) and t[holes, r] Sf (nh x nv x nel), then n^3 + 2 n^2
+    # complex MACs per n-hole determinant (the reduced closed form); 8 flops per complex MAC
     macs = 0.0
     for s in (0, 1):
         nel = trial.nup if s == 0 else trial.ndn
         nact = trial.orbmat[s].shape[0]
         nv = nact - nel
         nh = len({int(h) for n, e in trial.exc[s].items() for h in e[:, :n].ravel()})
-        macs += nel * nv * nel + nh * nact * nel + nh * nv * nel
-        macs += sum(len(e) * (3 * n ** 3 + 6 * n ** 2 + 3 * n) for n, e in trial.exc[s].items())
+        macs += nel * nv * nel + nh * nv * nel
+        macs += sum(len(e) * (n ** 3 + 2 * n ** 2) for n, e in trial.exc[s].items())
     flops = 8.0 * W * wl.Nc * macs
-    fp64 = fp64_peak_tflops(torch)
     achieved = flops / (phases["energy_measurement"] / 1000) / 1e12
-    roofline = {"kernel": "energy_measurement (excited_energy_tables_kernel ~80%)",
-                "bound": "fp64", "achieved": achieved, "peak": fp64, "unit": "TFLOP/s",
-                "frac": achieved / fp64, "traffic": None, "flops_per_launch": flops,
-                "peak_source": "cuBLAS DGEMM 8192^3 measured in this run"}
+    if prec == A.PREC_MIXED:
+        kernel, bound, peak = "excited_energy_groups_kernel ~73%", "latency", 74.5
+        peak_src = "nominal: 148 SMs x 128 FP32 multiply-adds x 1965 MHz (no FP32 entry in the " \
+                   "file of measured peaks)"
+    else:
+        kernel, bound, peak = "excited_energy_tables_kernel", "fp64", fp64_peak_tflops(torch)
+        peak_src = "cuBLAS DGEMM 8192^3 measured in this run"
+    roofline = {"kernel": f"energy_measurement ({kernel})", "bound": bound, "achieved": achieved,
+                "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
+                "flops_per_launch": flops, "peak_source": peak_src}
     e2e = None if args.no_e2e else _e2e(sim, W, wl.Nc, args.steps, args.warmup, world, prec)
     if rank == 0:
         line = {
