@@ -59,15 +59,16 @@ int fit_rows(int m) {
 // Time (cycles) of a single problem in a shape, up to what all shapes share.  A K tile of a CTA costs its
 // SM the DMMAs of the busiest scheduler and the fragment loads of all its warps (x), and takes no less
 // than the latency of a stage, which grows with the copies a thread issues for it; resident CTAs
-// overlap that latency, and what does not fit a wave adds another.  Clusters of four and eight leave
-// about a twelfth of the SMs unused.  The constants are fitted to 2200 timings of 42 problems
-// (1..1536 rows, 60..40000 columns, K = 57..4290).
+// overlap that latency, and what does not fit a wave adds another; a wave fills its ring first.  Clusters
+// of four and eight leave about a twelfth of the SMs unused.  The constants are fitted to timings of 114
+// problems in all shapes (1..2400 rows, 26..40000 columns, K = 35..4290; 61 of them from the steps and
+// energies of molecules and model systems).
 double model_time(const Shape& sh, int m, int n, int k, bool a_real, bool b_real) {
   const int w = sh.warps, tn = sh.tn, c = sh.split;
   const int frag_a = a_real ? 2 : 4, frag_b = b_real ? 2 : 4;  // wavefronts of a fragment load
   const int mma = a_real && b_real ? 1 : (a_real || b_real ? 2 : 4);
-  const double x = 0.6 * ((w + 3) / 4 * tn * 4 * mma * 16) + 2.2 * (w * 4 * (frag_a + tn * frag_b));
-  const double latency = 77.0 * (4 + (4 * tn + w - 1) / w) + 0.9 * x;
+  const double x = 0.6 * ((w + 3) / 4 * tn * 4 * mma * 16) + 1.6 * (w * 4 * (frag_a + tn * frag_b));
+  const double latency = 90.0 * (4 + (4 * tn + w - 1) / w) + 0.9 * x;
   const int ring = STAGES * 8 * (BK + 4) * (w * (a_real ? 8 : 16) + tn * (b_real ? 8 : 16));
   const int smem = (c > 1 ? std::max(ring, 64 * w * tn * 16) : ring) + 1024;
   const int resident = std::max(1, std::min(227 * 1024 / smem, 16 / w));
@@ -76,24 +77,24 @@ double model_time(const Shape& sh, int m, int n, int k, bool a_real, bool b_real
   const int waves = per_sm / resident, rest = per_sm - waves * resident;
   const double cycles = waves * std::max(resident * x, latency) +
                         (rest ? std::max(rest * x, latency) : 0.0);
-  return cycles * (((k + BK - 1) / BK + c - 1) / c) + (c > 1 ? 3000.0 : 0.0);
+  const int ktiles = ((k + BK - 1) / BK + c - 1) / c;
+  return cycles * (ktiles + STAGES - 1) + (c > 1 ? 3000.0 : 0.0);
 }
 
 // 64 x 64 tiles fill the SMs twice over
 bool many_tiles(int m, long n) { return ceil_div(m, 64) * long(ceil_div(n, 64)) >= 2 * NUM_SMS; }
 
-// The shape for a single problem of few tiles: the fitted one, or that of least time by the model if it
-// saves a twentieth.  K is split in two K tiles or more each, and not where there are many tiles.  On
-// the problems above and 61 that the steps and energies of molecules and model systems pose, the choice
-// is within 8% of the fastest of all shapes in the mean, and never more than 1.5% slower than the
-// fitted shape alone, which took 1.36 times the fastest in the mean: 1024 x 400 x 4160 (real B) in
-// tiles of 64 x 40 is 160 CTAs, two on 12 of the SMs and one on the others (462 us; in 32 x 32 333),
-// and 1 x 4096 x 200 one warp an SM (27.5 us; in 16 x 8 11).  More widths than these four cost the host
-// time (0.4 us for four) and gain 1%.
-Shape least_time(Shape fit, int m, int n, int k, bool a_real, bool b_real) {
+// The shape for a single problem of few tiles: the fitted one, or that of least time by the model if its
+// time is below `worth` of the fitted shape's.  K is split in two K tiles or more each, and not where
+// there are many tiles.  On the problems above the choice is within 7.5% of the fastest of all shapes in
+// the mean, and never more than 1.5% slower than the fitted shape, which alone takes 1.35 times the
+// fastest in the mean: 1024 x 400 x 4160 (real B) in tiles of 64 x 40 is 160 CTAs, two on 12 of the SMs
+// and one on the others (462 us; in 32 x 32 333), and 1 x 4096 x 200 one warp an SM (27.5 us; in 16 x 8
+// 11).  More widths than these four cost the host time (0.6 us for four) and gain 1%.
+Shape least_time(Shape fit, double worth, int m, int n, int k, bool a_real, bool b_real) {
   const int ktiles = ceil_div(k, BK);
   const bool may_split = !many_tiles(m, n);
-  double least = 0.95 * model_time(fit, m, n, k, a_real, b_real);
+  double least = worth * model_time(fit, m, n, k, a_real, b_real);
   for (int w = m >= 64 ? 4 : 1; w <= 8 && (w <= 2 || m > 4 * w); w *= 2)
     for (const int tn : {1, 2, 4, 7}) {
       if (n <= 8 * (tn - 1)) break;
@@ -113,11 +114,14 @@ Shape least_time(Shape fit, int m, int n, int k, bool a_real, bool b_real) {
 // The CTA shape: tiles fitted to m and n; then, where those are too few to give every SM one, the K
 // range of a single problem split over a cluster of up to 8 CTAs (each keeping at least 8 K tiles),
 // and the tiles halved down to 8 strips in all (below that the operand loads bound a tile).  For a
-// single problem of few tiles the model looks for a faster one.
+// single problem of few tiles the model looks for a faster one, by a twentieth; where the fitted tiles
+// give every SM two the waves cost less, and the gain has to stand out of the model's error (1024 x
+// 1600 x 10000, a force bias of the M = 200 system, was 2% slower in the tiles that it put at 0.93).
 Shape shape(int batch, int m, int n, int k, bool a_real, bool b_real) {
   Shape sh{fit_rows(m), fit_cols(n), 1};
   auto ctas = [&] { return long(ceil_div(m, 8 * sh.warps)) * ceil_div(n, 8 * sh.tn) * batch; };
   const bool few = batch == 1 && ctas() < 5 * NUM_SMS;
+  const double worth = ctas() < 2 * NUM_SMS ? 0.95 : 0.85;
   if (batch == 1 && ctas() < NUM_SMS)
     sh.split = std::max(1, std::min({8, int(NUM_SMS / ctas()), ceil_div(k, BK) / 8}));
   while (ctas() * sh.split < NUM_SMS && sh.warps * sh.tn > 8) {
@@ -126,7 +130,7 @@ Shape shape(int batch, int m, int n, int k, bool a_real, bool b_real) {
     else
       sh.warps = (sh.warps + 1) / 2;
   }
-  if (few) return least_time(sh, m, n, k, a_real, b_real);
+  if (few) return least_time(sh, worth, m, n, k, a_real, b_real);
   if (m > 65535l * 8 * sh.warps) sh.warps = 8;  // grid.y limit
   return sh;
 }
